@@ -131,8 +131,6 @@ struct dl_handle {
     double* f64[2];          // SoA populations [15][N], two buffers
     double* g64[2];
     double* mac64[2];        // [5][N]: phi, u1, u2, u3, p
-    double* rec64;           // derived records, [NREC][N]
-    int nrec;
     double* force64;         // [3][N]
 
     // reduced precision forms (FP32 / FP16 storage)
