@@ -36,109 +36,171 @@ struct SpArgs {
     double Nd;
 };
 
-__device__ __forceinline__ int modi(long long v, int n) { return (int)(((v % n) + n) % n); }
+// The sums of a wavenumber run over the grid in sequence, so parallelism comes
+// from the outputs, and the bound is the FP64 pipe (a warp's FP64 instruction
+// takes the SM 16 cycles): k = 0 adds v itself (its twiddle is exactly 1 + 0i),
+// table indices advance by k instead of by a division, and the loads of
+// several terms are in flight together. Measured at 128^3, kc = 3, before and
+// after (us): x stage 317 -> 239, y 117 -> 36, z 70 -> 14, energy 104 -> 6,
+// synthesis y 26.5 -> 22, x 289 -> 195.
 
-// x stage: a1[c][kx][y][z] = sum_x u e^{-i 2 pi kx x / nx}
-__global__ void sp_xstage(const SpArgs a) {
-    const int NK = 2 * a.K + 1;
-    long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const long long total = 3LL * NK * a.ny * a.nz;
-    if (t >= total) return;
-    const int z = (int)(t % a.nz);
-    long long r = t / a.nz;
-    const int y = (int)(r % a.ny);
-    r /= a.ny;
-    const int kxi = (int)(r % NK);
-    const int c = (int)(r / NK);
-    const int kx = kxi - a.K;
-    const double* u = a.u[c] + ((long long)z * a.ny + y) * a.nx;
-    double re = 0.0, im = 0.0;
-    for (int x = 0; x < a.nx; ++x) {
-        const int m = modi((long long)kx * x, a.nx);
-        const double v = u[x];
-        re = re + v * a.twx[2 * m];
-        im = im - v * a.twx[2 * m + 1];
-    }
-    double* d = a.a1 + 2 * ((((long long)c * NK + kxi) * a.ny + y) * a.nz + z);
-    d[0] = re;
-    d[1] = im;
+// m + k in [0, n), |k| < n
+__device__ __forceinline__ int step_mod(int m, int k, int n) {
+    m += k;
+    if (m >= n) m -= n;
+    if (m < 0) m += n;
+    return m;
+}
+// k x mod n for |k x| below 2^31
+__device__ __forceinline__ int mul_mod(int k, int x, int n) {
+    const int m = (k * x) % n;
+    return m < 0 ? m + n : m;
 }
 
-// y stage: a2[c][kx][ky][z] = sum_y a1 e^{-i 2 pi ky y / ny}
-__global__ void sp_ystage(const SpArgs a) {
+// x stage: a1[c][kx][y][z] = sum_x u e^{-i 2 pi kx x / nx}. A block takes 32
+// rows (one y, 32 z) of a component; its 2K warps take one kx != 0 each, and one
+// of them, another in each block, the plain sum of kx = 0 as well. The rows
+// come through shared memory, 32 columns at a time, so that the loads run along
+// x while every lane sums its own row in order.
+__global__ void sp_xstage(const SpArgs a, int nzb) {
+    __shared__ double tile[32][33];
+    const int NK = 2 * a.K + 1, nw = 2 * a.K;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, kx = warp < a.K ? warp - a.K : warp - a.K + 1;
+    const bool also0 = (int)(blockIdx.x % nw) == warp;
+    const int z0 = (int)(blockIdx.x % nzb) * 32, r = (int)(blockIdx.x / nzb), y = r % a.ny, c = r / a.ny;
+    const double* u = a.u[c] + (long long)y * a.nx;
+    const double2* tw = reinterpret_cast<const double2*>(a.twx);
+    double re = 0.0, im = 0.0, s0 = 0.0;
+    int m = 0;
+    for (int x0 = 0; x0 < a.nx; x0 += 32) {
+        const int w = min(32, a.nx - x0);
+        __syncthreads();
+        for (int r = warp; r < 32; r += nw)
+            if (z0 + r < a.nz && lane < w) tile[r][lane] = __ldg(u + (long long)(z0 + r) * a.ny * a.nx + x0 + lane);
+        __syncthreads();
+        const double* row = tile[lane];
+        int x = 0;
+        for (; x + 8 <= w; x += 8) {
+            double2 t[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                t[k] = __ldg(tw + m);
+                m = step_mod(m, kx, a.nx);
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const double v = row[x + k];
+                re = re + v * t[k].x;
+                im = im - v * t[k].y;
+            }
+        }
+        for (; x < w; ++x) {
+            const double2 t = __ldg(tw + m);
+            re = re + row[x] * t.x;
+            im = im - row[x] * t.y;
+            m = step_mod(m, kx, a.nx);
+        }
+        if (also0)
+            for (x = 0; x < w; ++x) s0 = s0 + row[x];
+    }
+    if (z0 + lane >= a.nz) return;
+    double2* d = reinterpret_cast<double2*>(a.a1) + ((long long)c * NK * a.ny + y) * a.nz + z0 + lane;
+    const long long plane = (long long)a.ny * a.nz;
+    d[(kx + a.K) * plane] = make_double2(re, im);
+    if (also0) d[a.K * plane] = make_double2(s0, 0.0);
+}
+
+// y stage: a2[c][kx][ky][z] = sum_y a1 e^{-i 2 pi ky y / ny}; real and
+// imaginary part are two threads' sums (block: 32 z x 2 parts)
+__global__ void __launch_bounds__(64) sp_ystage(const SpArgs a) {
+    constexpr int B = 16;  // terms in flight
     const int NK = 2 * a.K + 1;
-    long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const long long total = 3LL * NK * NK * a.nz;
-    if (t >= total) return;
-    const int z = (int)(t % a.nz);
-    long long r = t / a.nz;
-    const int kyi = (int)(r % NK);
-    r /= NK;
-    const int kxi = (int)(r % NK);
-    const int c = (int)(r / NK);
+    const int z = blockIdx.x * 32 + (threadIdx.x & 31), part = threadIdx.x >> 5;
+    const int kxi = blockIdx.y / NK, kyi = blockIdx.y % NK, c = blockIdx.z;
+    if (z >= a.nz) return;
     const int ky = kyi - a.K;
-    double re = 0.0, im = 0.0;
-    for (int y = 0; y < a.ny; ++y) {
-        const int m = modi((long long)ky * y, a.ny);
-        const double* v = a.a1 + 2 * ((((long long)c * NK + kxi) * a.ny + y) * a.nz + z);
-        const double cy_ = a.twy[2 * m], sy_ = a.twy[2 * m + 1];
-        re = re + (v[0] * cy_ + v[1] * sy_);
-        im = im + (v[1] * cy_ - v[0] * sy_);
+    const double2* v = reinterpret_cast<const double2*>(a.a1) + ((long long)c * NK + kxi) * a.ny * a.nz + z;
+    const double2* tw = reinterpret_cast<const double2*>(a.twy);
+    double s = 0.0;
+    int m = 0;
+    for (int y0 = 0; y0 < a.ny; y0 += B) {
+        double2 t[B], e[B];
+#pragma unroll
+        for (int k = 0; k < B; ++k) {
+            const int y = min(y0 + k, a.ny - 1);
+            t[k] = __ldg(v + (long long)y * a.nz);
+            if (ky != 0) e[k] = __ldg(tw + m);
+            m = step_mod(m, ky, a.ny);
+        }
+        if (ky == 0) {
+#pragma unroll
+            for (int k = 0; k < B; ++k)
+                if (y0 + k < a.ny) s = s + (part ? t[k].y : t[k].x);
+        } else {
+#pragma unroll
+            for (int k = 0; k < B; ++k) {
+                // re: v0 cos + v1 sin; im: v1 cos - v0 sin
+                const double p = part ? t[k].y : t[k].x, q = part ? -t[k].x : t[k].y;
+                if (y0 + k < a.ny) s = s + (p * e[k].x + q * e[k].y);
+            }
+        }
     }
-    double* d = a.a2 + 2 * ((((long long)c * NK + kxi) * NK + kyi) * a.nz + z);
-    d[0] = re;
-    d[1] = im;
+    a.a2[2 * ((((long long)c * NK + kxi) * NK + kyi) * a.nz + z) + part] = s;
 }
 
-// z stage: uh[c][kx][ky][kz] = (sum_z a2 e^{-i 2 pi kz z / nz}) / N, kz = 0..K
-__global__ void sp_zstage(const SpArgs a) {
-    const int NK = 2 * a.K + 1;
-    long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const long long total = 3LL * NK * NK * (a.K + 1);
-    if (t >= total) return;
-    const int kz = (int)(t % (a.K + 1));
-    long long r = t / (a.K + 1);
-    const int kyi = (int)(r % NK);
-    r /= NK;
-    const int kxi = (int)(r % NK);
-    const int c = (int)(r / NK);
-    double re = 0.0, im = 0.0;
-    for (int z = 0; z < a.nz; ++z) {
-        const int m = (int)(((long long)kz * z) % a.nz);
-        const double* v = a.a2 + 2 * ((((long long)c * NK + kxi) * NK + kyi) * a.nz + z);
-        const double cz_ = a.twz[2 * m], sz_ = a.twz[2 * m + 1];
-        re = re + (v[0] * cz_ + v[1] * sz_);
-        im = im + (v[1] * cz_ - v[0] * sz_);
+// z stage: uh[c][kx][ky][kz] = (sum_z a2 e^{-i 2 pi kz z / nz}) / N, kz = 0..K.
+// One warp per value: the lanes form the terms of 32 z at once, lane 0 adds the
+// real and lane 16 the imaginary ones in order.
+__global__ void __launch_bounds__(32) sp_zstage(const SpArgs a) {
+    const int lane = threadIdx.x;
+    const int kz = blockIdx.x % (a.K + 1), r = blockIdx.x / (a.K + 1);  // r = (c NK + kxi) NK + kyi
+    const double2* v = reinterpret_cast<const double2*>(a.a2) + (long long)r * a.nz;
+    double s = 0.0;
+    for (int z0 = 0; z0 < a.nz; z0 += 32) {
+        const int w = min(32, a.nz - z0);
+        double pr = 0.0, pi = 0.0;
+        if (lane < w) {
+            const double2 t = __ldg(v + z0 + lane);
+            const double2 e = __ldg(reinterpret_cast<const double2*>(a.twz) + (int)(((long long)kz * (z0 + lane)) % a.nz));
+            pr = t.x * e.x + t.y * e.y;
+            pi = t.y * e.x - t.x * e.y;
+        }
+        // (terms past w are +0 and are not added: -0 + 0 would be +0)
+#pragma unroll
+        for (int k = 0; k < 32; ++k) {
+            const double tr = __shfl_sync(0xffffffffu, pr, k), ti = __shfl_sync(0xffffffffu, pi, k);
+            const double t = lane < 16 ? tr : ti;
+            if (k < w) s = s + t;
+        }
     }
-    double* d = a.uh + 2 * ((((long long)c * NK + kxi) * NK + kyi) * (a.K + 1) + kz);
-    d[0] = re / a.Nd;
-    d[1] = im / a.Nd;
+    if (lane == 0 || lane == 16) a.uh[2 * ((long long)r * (a.K + 1) + kz) + (lane >> 4)] = s / a.Nd;
 }
 
 // band energy in the reference's loop order (k3 outer, then k2, then k1, each
-// in FFT index order) and the coefficient 0.5 eps / E; one thread.
-__global__ void sp_energy(const SpArgs a) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const int NK = 2 * a.K + 1;
-    double energy = 0.0;
-    for (int k3 = 0; k3 <= a.K; ++k3)
-        for (int i2 = 0; i2 < a.ny; ++i2) {
-            const int k2 = (i2 >= a.ny / 2 + 1) ? i2 - a.ny : i2;
-            if (k2 < -a.K || k2 > a.K) continue;
-            for (int i1 = 0; i1 < a.nx; ++i1) {
-                const int k1 = (i1 >= a.nx / 2 + 1) ? i1 - a.nx : i1;
-                if (k1 < -a.K || k1 > a.K) continue;
-                const int kk = k1 * k1 + k2 * k2 + k3 * k3;
-                if (kk < 1 || kk >= a.kc2) continue;
-                double e[3];
-                for (int c = 0; c < 3; ++c) {
-                    const double* v = a.uh + 2 * ((((long long)c * NK + (k1 + a.K)) * NK + (k2 + a.K)) * (a.K + 1) + k3);
-                    e[c] = v[0] * v[0] + v[1] * v[1];
-                }
-                const double w = 2.0 < (double)k3 + 1.0 ? 2.0 : (double)k3 + 1.0;
-                energy = energy + 0.5 * (e[0] + e[1] + e[2]) * w;
-            }
+// in FFT index order 0 .. K, -K .. -1) and the coefficient 0.5 eps / E: one
+// block forms the terms, one thread adds them. MAXT: terms of the largest band
+// (K = 4), all of the box 0..K x (2K+1)^2.
+constexpr int SP_MAXT = 5 * 9 * 9;
+__global__ void __launch_bounds__(256) sp_energy(const SpArgs a) {
+    __shared__ double term[SP_MAXT];
+    const int NK = 2 * a.K + 1, n = NK * NK * (a.K + 1);
+    for (int t = threadIdx.x; t < n; t += blockDim.x) {
+        const int i1 = t % NK, r = t / NK, i2 = r % NK, k3 = r / NK;
+        const int k1 = i1 <= a.K ? i1 : i1 - NK, k2 = i2 <= a.K ? i2 : i2 - NK;
+        const int kk = k1 * k1 + k2 * k2 + k3 * k3;
+        double e[3];
+        for (int c = 0; c < 3; ++c) {
+            const double* v = a.uh + 2 * ((((long long)c * NK + (k1 + a.K)) * NK + (k2 + a.K)) * (a.K + 1) + k3);
+            e[c] = v[0] * v[0] + v[1] * v[1];
         }
+        const double w = 2.0 < (double)k3 + 1.0 ? 2.0 : (double)k3 + 1.0;
+        // outside the band: +0, which changes no sum of squares
+        term[t] = (kk < 1 || kk >= a.kc2) ? 0.0 : 0.5 * (e[0] + e[1] + e[2]) * w;
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    double energy = 0.0;
+    for (int t = 0; t < n; ++t) energy = energy + term[t];
     a.st->sp_energy = energy;
     a.st->sp_coef = a.half_eps / energy;
 }
@@ -186,39 +248,61 @@ __global__ void sp_synth_y(const SpArgs a) {
     r /= a.ny;
     const int kxi = (int)(r % NK);
     const int c = (int)(r / NK);
+    const double2* b1 = reinterpret_cast<const double2*>(a.b1) + ((long long)c * NK + kxi) * NK * a.nz + z;
     double re = 0.0, im = 0.0;
+    int m = mul_mod(-a.K, y, a.ny);
     for (int kyi = 0; kyi < NK; ++kyi) {
-        const int ky = kyi - a.K;
-        const double* v = a.b1 + 2 * ((((long long)c * NK + kxi) * NK + kyi) * a.nz + z);
-        const int m = modi((long long)ky * y, a.ny);
-        const double cy_ = a.twy[2 * m], sy_ = a.twy[2 * m + 1];
-        re = re + (v[0] * cy_ - v[1] * sy_);
-        im = im + (v[0] * sy_ + v[1] * cy_);
+        const double2 v = __ldg(b1 + (long long)kyi * a.nz);
+        if (kyi == a.K) {
+            re = re + v.x;
+            im = im + v.y;
+        } else {
+            const double2 e = __ldg(reinterpret_cast<const double2*>(a.twy) + m);
+            re = re + (v.x * e.x - v.y * e.y);
+            im = im + (v.x * e.y + v.y * e.x);
+        }
+        m = step_mod(m, y, a.ny);
     }
-    double* d = a.b2 + 2 * ((((long long)c * NK + kxi) * a.ny + y) * a.nz + z);
-    d[0] = re;
-    d[1] = im;
+    reinterpret_cast<double2*>(a.b2)[(((long long)c * NK + kxi) * a.ny + y) * a.nz + z] = make_double2(re, im);
 }
 
-__global__ void sp_synth_x(const SpArgs a) {
-    const int NK = 2 * a.K + 1;
-    long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const long long N = (long long)a.nx * a.ny * a.nz;
-    if (t >= 3 * N) return;
-    const int c = (int)(t / N);
-    const long long s = t - c * N;
-    const int x = (int)(s % a.nx);
-    const long long r = s / a.nx;
-    const int y = (int)(r % a.ny);
-    const int z = (int)(r / a.ny);
-    double re = 0.0;
-    for (int kxi = 0; kxi < NK; ++kxi) {
-        const int kx = kxi - a.K;
-        const double* v = a.b2 + 2 * ((((long long)c * NK + kxi) * a.ny + y) * a.nz + z);
-        const int m = modi((long long)kx * x, a.nx);
-        re = re + (v[0] * a.twx[2 * m] - v[1] * a.twx[2 * m + 1]);
+// a warp's 32 sites along x share their row's coefficients; a thread takes the
+// three components of its site (block: 32 x by 4 rows of the flattened y, z)
+template <int K>
+__global__ void __launch_bounds__(128) sp_synth_x(const SpArgs a, int nxb) {
+    constexpr int NK = 2 * K + 1;
+    const int x = (int)(blockIdx.x % nxb) * 32 + (threadIdx.x & 31);
+    const long long r = (long long)(blockIdx.x / nxb) * 4 + (threadIdx.x >> 5);
+    const int z = (int)(r / a.ny), y = (int)(r - (long long)z * a.ny);
+    if (x >= a.nx || z >= a.nz) return;
+    const double2* b2 = reinterpret_cast<const double2*>(a.b2) + (long long)y * a.nz + z;
+    const long long plane = (long long)a.ny * a.nz;
+    double2 e[NK];
+    int m = mul_mod(-K, x, a.nx);
+#pragma unroll
+    for (int k = 0; k < NK; ++k) {
+        if (k != K) e[k] = __ldg(reinterpret_cast<const double2*>(a.twx) + m);
+        m = step_mod(m, x, a.nx);
     }
-    a.fo[c][s] = re;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        double2 v[NK];
+#pragma unroll
+        for (int k = 0; k < NK; ++k) v[k] = __ldg(b2 + (c * NK + k) * plane);
+        double f = v[0].x * e[0].x - v[0].y * e[0].y;
+#pragma unroll
+        for (int k = 1; k < NK; ++k) f = k == K ? f + v[k].x : f + (v[k].x * e[k].x - v[k].y * e[k].y);
+        a.fo[c][r * a.nx + x] = f;
+    }
+}
+
+static void launch_synth_x(const SpArgs& a, cudaStream_t s) {
+    const int nxb = (a.nx + 31) / 32;
+    const unsigned g = (unsigned)(nxb * (((long long)a.ny * a.nz + 3) / 4));
+    if (a.K == 1) sp_synth_x<1><<<g, 128, 0, s>>>(a, nxb);
+    else if (a.K == 2) sp_synth_x<2><<<g, 128, 0, s>>>(a, nxb);
+    else if (a.K == 3) sp_synth_x<3><<<g, 128, 0, s>>>(a, nxb);
+    else sp_synth_x<4><<<g, 128, 0, s>>>(a, nxb);
 }
 
 // FP32 forms: the x stage with one warp per (y, z) row (lanes over x, FP32
@@ -460,15 +544,14 @@ int spectral_force_fp64(dl_handle* h, const double* u1, const double* u2, const 
     a.fo[1] = fy;
     a.fo[2] = fz;
     const int NK = 2 * a.K + 1;
-    const long long N = (long long)h->N;
     cudaStream_t s = h->stream;
-    DL_LAUNCH(h, false, sp_xstage<<<nb(3LL * NK * h->ny * h->nz, 128), 128, 0, s>>>(a));
-    DL_LAUNCH(h, false, sp_ystage<<<nb(3LL * NK * NK * h->nz, 128), 128, 0, s>>>(a));
-    DL_LAUNCH(h, false, sp_zstage<<<nb(3LL * NK * NK * (a.K + 1), 64), 64, 0, s>>>(a));
-    DL_LAUNCH(h, false, sp_energy<<<1, 32, 0, s>>>(a));
+    DL_LAUNCH(h, false, (sp_xstage<<<(unsigned)((h->nz + 31) / 32 * 3LL * h->ny), 64 * a.K, 0, s>>>(a, (h->nz + 31) / 32)));
+    DL_LAUNCH(h, false, (sp_ystage<<<dim3((h->nz + 31) / 32, NK * NK, 3), 64, 0, s>>>(a)));
+    DL_LAUNCH(h, false, (sp_zstage<<<3 * NK * NK * (a.K + 1), 32, 0, s>>>(a)));
+    DL_LAUNCH(h, false, (sp_energy<<<1, 256, 0, s>>>(a)));
     DL_LAUNCH(h, false, sp_synth_z<<<nb(3LL * NK * NK * h->nz, 128), 128, 0, s>>>(a));
     DL_LAUNCH(h, false, sp_synth_y<<<nb(3LL * NK * h->ny * h->nz, 128), 128, 0, s>>>(a));
-    DL_LAUNCH(h, false, sp_synth_x<<<nb(3 * N, 256), 256, 0, s>>>(a));
+    DL_LAUNCH(h, false, launch_synth_x(a, s));
     DL_CUDA(h, cudaGetLastError());
     return DL_OK;
 }
@@ -482,8 +565,8 @@ int spectral_project_f32(dl_handle* h, const float* u1, const float* u2, const f
     const long long rows = (long long)h->ny * h->nz;
     DL_LAUNCH(h, false, sp_xstage_f32<<<nb(rows * 32, 256), 256, 0, s>>>(u1, u2, u3, a.a1, h->nx, h->ny, h->nz, a.K,
                                                                         h->sp.d_twxf));
-    DL_LAUNCH(h, false, sp_ystage<<<nb(3LL * NK * NK * h->nz, 128), 128, 0, s>>>(a));
-    DL_LAUNCH(h, false, sp_zstage<<<nb(3LL * NK * NK * (a.K + 1), 64), 64, 0, s>>>(a));
+    DL_LAUNCH(h, false, (sp_ystage<<<dim3((h->nz + 31) / 32, NK * NK, 3), 64, 0, s>>>(a)));
+    DL_LAUNCH(h, false, (sp_zstage<<<3 * NK * NK * (a.K + 1), 32, 0, s>>>(a)));
     DL_CUDA(h, cudaGetLastError());
     return DL_OK;
 }
@@ -506,7 +589,7 @@ int spectral_adjoint_f32(dl_handle* h, const float* lf1, const float* lf2, const
     fill_sp(h, a);
     cudaStream_t s = h->stream;
     const long long N = (long long)h->N;
-    DL_LAUNCH(h, false, sp_energy<<<1, 32, 0, s>>>(a));
+    DL_LAUNCH(h, false, (sp_energy<<<1, 256, 0, s>>>(a)));
     DL_LAUNCH(h, false, sp_adj_combine<<<1, 256, 0, s>>>(a, sp.d_lh));
     DL_LAUNCH(h, false, sp_synth_z<<<nb(3LL * NK * NK * h->nz, 128), 128, 0, s>>>(a));
     DL_LAUNCH(h, false, sp_synth_y<<<nb(3LL * NK * h->ny * h->nz, 128), 128, 0, s>>>(a));
@@ -526,9 +609,9 @@ int spectral_force_f32(dl_handle* h, const float* u1, const float* u2, const flo
     const long long rows = (long long)h->ny * h->nz;
     DL_LAUNCH(h, false, sp_xstage_f32<<<nb(rows * 32, 256), 256, 0, s>>>(u1, u2, u3, a.a1, h->nx, h->ny, h->nz, a.K,
                                                                         h->sp.d_twxf));
-    DL_LAUNCH(h, false, sp_ystage<<<nb(3LL * NK * NK * h->nz, 128), 128, 0, s>>>(a));
-    DL_LAUNCH(h, false, sp_zstage<<<nb(3LL * NK * NK * (a.K + 1), 64), 64, 0, s>>>(a));
-    DL_LAUNCH(h, false, sp_energy<<<1, 32, 0, s>>>(a));
+    DL_LAUNCH(h, false, (sp_ystage<<<dim3((h->nz + 31) / 32, NK * NK, 3), 64, 0, s>>>(a)));
+    DL_LAUNCH(h, false, (sp_zstage<<<3 * NK * NK * (a.K + 1), 32, 0, s>>>(a)));
+    DL_LAUNCH(h, false, (sp_energy<<<1, 256, 0, s>>>(a)));
     DL_LAUNCH(h, false, sp_synth_z<<<nb(3LL * NK * NK * h->nz, 128), 128, 0, s>>>(a));
     DL_LAUNCH(h, false, sp_synth_y<<<nb(3LL * NK * h->ny * h->nz, 128), 128, 0, s>>>(a));
     DL_LAUNCH(h, false, sp_synth_x_f32<<<nb(N, 256), 256, 0, s>>>(a.b2, fx, fy, fz, h->nx, h->ny, h->nz, a.K,
