@@ -471,7 +471,7 @@ __global__ void __launch_bounds__(256) moments_fp64(const Fp64Args a) {
     if (!STEP) return;
     // NaN is skipped by the reference's comparisons; exclude it here as well
     const bool in = active && !nan_bits(ph);
-    minmax_block_and_finalize<double>(a.st, in ? ph : INFINITY, in ? ph : -INFINITY, a.maco, 0.0, N, a.phi1, a.phi2,
+    minmax_block_and_finalize<double, true>(a.st, in ? ph : INFINITY, in ? ph : -INFINITY, a.maco, 0.0, N, a.phi1, a.phi2,
                                       bad, a.step, gridDim.x);
 }
 

@@ -933,8 +933,8 @@ __device__ __forceinline__ void push_body(const PushArgs& pa, float* smem, int b
         spectral_block_done(a, smem, nblk);
     }
     if constexpr (SETTLE) {
-        minmax_block_and_finalize<float>(a.st, (double)bmin, (double)bmax, a.maco, a.phi1, a.N, (double)a.phi1,
-                                         (double)a.phi2, bad, a.step, nblk);
+        minmax_block_and_finalize<float, true>(a.st, (double)bmin, (double)bmax, a.maco, a.phi1, a.N, (double)a.phi1,
+                                               (double)a.phi2, bad, a.step, nblk);
     } else {
         push_minmax(a, bmin, bmax, bad, nblk);
     }
