@@ -105,10 +105,6 @@ struct FastSpectral {
 
 }  // namespace dl
 
-// z planes one block of the fused kernel marches by default: the autotuner's
-// choice for the 128^3 two-phase workloads in the FP32 and FP16 forms
-constexpr int DL_DEFAULT_LZ = 32;
-
 struct dl_handle {
     dl_params P;
     int nx, ny, nz;
@@ -138,7 +134,9 @@ struct dl_handle {
     void* gs[2];
     float* mac32[2];         // [5][N]: phi - phi1, u1, u2, u3, p - 1/3
     float* force32;          // [3][N]
-    int lz;                  // z planes per block of the fused kernel (0: DL_DEFAULT_LZ, at most nz)
+    int lz;                  // z planes per block of the fused kernel (0: chosen by march_planes)
+    int lz_auto[3];          // that choice by prologue class (0: not made yet)
+    int lz_settle[3];        // the same of a settle launch
     int l2_prefetch;         // fused kernel: bulk L2 prefetch of the next plane's pulls
     int sp_pipeline;         // single-phase kernel: next plane's pulls held in registers
     int proj_in_step;        // band forcing: projection of the new u inside the fused step (else its own launch)
@@ -217,6 +215,8 @@ void push_args_at(dl_handle* h, int k, void* out);
 int launch_push_batched(dl_handle* h0, const void* table, int nm, const int4* items, int nitems,
                         const unsigned* nblk, unsigned* counter, int grid, cudaStream_t s);
 int fast_prepare_force(dl_handle* h, int mode);
+int effective_lz(dl_handle* h);  // z planes per block of the next step
+int settle_lz(dl_handle* h);     // of a settle launch
 int spectral_project_f32(dl_handle* h, const float* d_u1, const float* d_u2, const float* d_u3);
 int spectral_adjoint_f32(dl_handle* h, const float* d_lf1, const float* d_lf2, const float* d_lf3, const float* d_u1,
                          const float* d_u2, const float* d_u3, float* d_lu1, float* d_lu2, float* d_lu3);

@@ -719,6 +719,24 @@ __global__ void __launch_bounds__(PROJ_NT, 4) sp_project_fast(const FastArgs a) 
     project_rows(a, blockIdx.x * W + (threadIdx.x >> 5), gridDim.x * W, a.ny * a.nz, gridDim.x);
 }
 
+// the projection of the fused step as a launch of its own, over chunks of
+// BAND_CHUNK planes whatever the step's lz: the same sums in the same order as
+// a step whose blocks march BAND_CHUNK planes. FP16 storage turns any change of
+// rounding in the force into one FP16 quantum here and there, which spreads, so
+// its band sums must not depend on how the step is cut.
+constexpr int BAND_CHUNK = 32;
+__global__ void __launch_bounds__(NT) project_chunks(const FastArgs a) {
+    __shared__ __align__(16) float scr[PT_SCRATCH];
+    __shared__ float2 s_tx[SNK * EX1], s_ty[SNK * EY1];
+    const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
+    const int gxd = x0 + threadIdx.x % TX, gyd = y0 + threadIdx.x / TX;
+    const int z0 = blockIdx.z * BAND_CHUNK, z1 = min(z0 + BAND_CHUNK, a.nz);
+    tile_twiddles(a, s_tx, s_ty, x0, y0);
+    project_tile(a, scr, s_tx, s_ty, gxd, gyd, z0, z1, gxd < a.nx && gyd < a.ny,
+                 blockIdx.x + 3 * blockIdx.y + 5 * blockIdx.z);
+    spectral_block_done(a, scr, gridDim.x * gridDim.y * gridDim.z);
+}
+
 // ---- initial populations f = feq, g = geq at every site (ini :244-251) -------
 template <typename ST, bool RES>
 __global__ void __launch_bounds__(256) init_fast(const FastArgs a) {
@@ -894,16 +912,101 @@ static size_t smem_bytes() {
     return sizeof(float) * (size_t)fused_smem_floats(LES, FMODE == F_SPECTRAL, FMODE != F_NONE, SP);
 }
 
+int sm_count(dl_handle* h) {
+    static int sms_of[64] = {0};
+    int& sms = sms_of[h->device & 63];
+    if (sms == 0 && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess) sms = 152;
+    return sms;
+}
+
+// ---- z planes per block ----------------------------------------------------
+// A block marches lz planes of its 32 x 8 column, two blocks to an SM. Its time
+// in units of one plane with both slots of the SM taken is prol + lz; alone on
+// its SM it takes 0.55 per plane (and half as much again for the prologue).
+// prol is 1 plane without band forcing (two ring planes, index tables), 2.5
+// with it (force tables, projection), 5 for the single-phase step, whose
+// planes are cheap. A launch is full waves of 2 x SMs blocks and a rest; the
+// rest costs a lone block's time when nothing ran before it on its SM, but
+// 0.9 of a full block's otherwise (the waves do not end together). The
+// candidates split nz evenly. Measured (us per step, at the constant 32 that
+// this replaces / at the chosen lz): FP32 LES and band forcing 32^3 122 / 24
+// (lz 1), 64^3 122 / 42 (4), 96^3 135 / 88 (12), 128^3 188 / 188 (32), 256^3
+// 1315 / 1289 (37); shear droplet 32^3 61 / 10, 64^3 69 / 20; pull form 96^3
+// 166 / 92; FP16 96^3 162 / 100. Over 13 shapes and five step variants the
+// choice is within 5 % of the best of a sweep.
+static double march_cost(int lz, const dl_handle* h, int sms, double prol) {
+    const long long blocks =
+        (long long)((h->nx + TX - 1) / TX) * ((h->ny + TY - 1) / TY) * ((h->nz + lz - 1) / lz);
+    const long long full = blocks / (2 * sms), rest = blocks % (2 * sms);
+    const double both = prol + lz, alone = 1.5 * prol + 0.55 * lz;
+    const double last = rest == 0 ? 0.0 : rest > sms ? both : full ? std::max(alone, 0.9 * both) : alone;
+    return (double)full * both + last;
+}
+
+static int march_planes(const dl_handle* h, int sms, double prol) {
+    int best = h->nz;
+    double cost = march_cost(best, h, sms, prol);
+    for (int c = 2; c <= h->nz; ++c) {
+        const int lz = (h->nz + c - 1) / c;
+        if (lz == best) continue;
+        const double t = march_cost(lz, h, sms, prol);
+        if (t < 0.999 * cost) {
+            cost = t;
+            best = lz;
+        }
+    }
+    return best;
+}
+
+static int prologue_class(const dl_handle* h) { return force_fmode(h) != F_SPECTRAL ? 0 : h->single ? 2 : 1; }
+static const double PROLOGUE_PLANES[3] = {1.0, 2.5, 5.0};
+
+// FP16 storage with band forcing: another lz than BAND_CHUNK needs the
+// projection as a launch of its own (project_chunks), about CHUNK_LAUNCH planes'
+// time (it hides no latency behind a march); it pays on small domains
+// (us per step at lz 32 before / now: 32^3 127 / 32, 64^3 133 / 51, 96^3
+// 165 / 107, 256^3 1525 / 1485)
+constexpr double CHUNK_LAUNCH = 2.0;
+static bool band_fp16(const dl_handle* h) { return h->form == DL_FORM_FP16 && force_fmode(h) == F_SPECTRAL; }
+
+int effective_lz(dl_handle* h) {
+    if (h->lz > 0) return h->lz;
+    const int c = prologue_class(h);
+    if (h->lz_auto[c] == 0) {
+        const int sms = sm_count(h);
+        const double prol = PROLOGUE_PLANES[c];
+        int lz = march_planes(h, sms, prol);
+        const int chunk = std::min(h->nz, BAND_CHUNK);
+        if (band_fp16(h) && march_cost(chunk, h, sms, prol) <= march_cost(lz, h, sms, prol) + CHUNK_LAUNCH)
+            lz = chunk;
+        h->lz_auto[c] = lz;
+    }
+    return h->lz_auto[c];
+}
+
+// z planes per block of a settle: it runs alone on its stream whatever the
+// steps' lz is (an ensemble's members settle one after another), and a block
+// has no ring planes to load, only the force tables to build
+int settle_lz(dl_handle* h) {
+    const int c = prologue_class(h);
+    if (h->lz_settle[c] == 0) h->lz_settle[c] = march_planes(h, sm_count(h), c ? 3.0 : 0.5);
+    return h->lz_settle[c];
+}
+
+// the step's band projection is project_chunks instead of the fused step's own
+static bool chunked_projection(dl_handle* h) {
+    return band_fp16(h) && h->proj_in_step && h->lz == 0 && effective_lz(h) != std::min(h->nz, BAND_CHUNK);
+}
+
 void fill_fast(dl_handle* h, FastArgs& a) {
     const dl_params& P = h->P;
     memset(&a, 0, sizeof(a));
     a.nx = h->nx;
     a.ny = h->ny;
     a.nz = h->nz;
-    a.lz = h->lz > 0 ? h->lz : std::min(h->nz, DL_DEFAULT_LZ);
+    a.lz = effective_lz(h);
     a.l2_prefetch = h->l2_prefetch;
-    a.proj_in_step = h->proj_in_step;
-
+    a.proj_in_step = h->proj_in_step && !chunked_projection(h);
     a.N = (long long)h->N;
     a.st = h->d_state;
     a.phi1 = (float)P.phi1;
@@ -1012,7 +1115,6 @@ int fast_alloc(dl_handle* h) {
         DL_CUDA(h, cudaMemsetAsync(h->gs[k], 0, es * Q * N, h->stream));
         DL_CUDA(h, cudaMemsetAsync(h->mac32[k], 0, sizeof(float) * 5 * N, h->stream));
     }
-    if (h->lz <= 0) h->lz = std::min(h->nz, DL_DEFAULT_LZ);
     return fast_spectral_alloc(h);
 }
 
@@ -1111,16 +1213,15 @@ static int fast_spectral_project(dl_handle* h) {
 
 static const int PROJ_ROWS = 64;  // rows of the band projection per block (batched ensembles)
 
-static int sm_count(dl_handle* h) {
-    static int sms_of[64] = {0};
-    int& sms = sms_of[h->device & 63];
-    if (sms == 0 && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess) sms = 152;
-    return sms;
-}
-
 // band projection launch: four blocks on every SM (the register limit), one
 // wave; fewer blocks when there are fewer rows than warps
 static int launch_projection(dl_handle* h, const FastArgs& a) {
+    if (chunked_projection(h)) {
+        const dim3 grid((a.nx + TX - 1) / TX, (a.ny + TY - 1) / TY, (a.nz + BAND_CHUNK - 1) / BAND_CHUNK);
+        DL_LAUNCH(h, false, (project_chunks<<<grid, NT, 0, h->stream>>>(a)));
+        DL_CUDA(h, cudaGetLastError());
+        return DL_OK;
+    }
     const long long rows = (long long)a.ny * a.nz;
     const int sms = sm_count(h);
     const long long need = (rows + PROJ_NT / 32 - 1) / (PROJ_NT / 32);
@@ -1325,7 +1426,8 @@ struct BatchImpl {
     int2* d_pitems;         // projection work items (member, row block)
     unsigned* d_pnblk;      // projection blocks per member
     int npitems;
-    int lz, bps, use_graph;
+    int lz, bps, use_graph; // lz 0: chosen by batch_lz
+    int lz_auto[3];         // that choice by prologue class (0: not made yet)
     int persistent;         // 1: one persistent launch per step over all members; 0: the members' own steps, concurrent
     int nworkers;           // concurrent mode: worker streams (created on first use)
     cudaStream_t workers[BATCH_WORKERS];
@@ -1343,6 +1445,38 @@ struct BatchImpl {
     void* d_ptable;
     unsigned* d_counter;    // push form: the launch's next work item
 };
+
+// One lz for all members. Their launches overlap, so there are no common waves:
+// the cost is every block's planes and prologue (4.5 planes here) over the
+// 2 x SMs slots, and a quarter of a block for the end of the step, where few
+// are left; at least one block's time. Measured (us per step at the constant 32
+// before / at the choice): 64 members of 48^3 .. 96^3 1884 / 1845, 16 members
+// 624 / 612, two of 96^3 183 / 149. FP16 members with band forcing keep
+// BAND_CHUNK (its sums are grouped by chunk, see project_chunks).
+static int batch_lz(BatchImpl* b) {
+    if (b->lz > 0) return b->lz;
+    const int c = prologue_class(b->mem[0]);
+    if (b->lz_auto[c]) return b->lz_auto[c];
+    int nzmax = 1;
+    for (int m = 0; m < b->nm; ++m) nzmax = std::max(nzmax, b->mem[m]->nz);
+    int best = BAND_CHUNK;
+    double cost = INFINITY;
+    for (int k = (nzmax + 63) / 64; k <= nzmax && !band_fp16(b->mem[0]); ++k) {  // at most 64 planes
+        const int lz = (nzmax + k - 1) / k;
+        double planes = 0.0;
+        for (int m = 0; m < b->nm; ++m) {
+            const dl_handle* h = b->mem[m];
+            const int l = std::min(lz, h->nz);
+            planes += (double)((h->nx + TX - 1) / TX) * ((h->ny + TY - 1) / TY) * (h->nz + 4.5 * ((h->nz + l - 1) / l));
+        }
+        const double t = std::max(planes / (2 * b->sms) + 0.25 * lz, lz + 4.5);
+        if (t < 0.999 * cost) {
+            cost = t;
+            best = lz;
+        }
+    }
+    return b->lz_auto[c] = best;
+}
 
 template <typename ST, bool RES, bool LES, int FMODE>
 static int launch_batched_t(dl_handle* h0, BatchImpl* b, int k) {
@@ -1396,7 +1530,7 @@ int batch_create(dl_handle** members, int nm, void** out) {
     b->nm = nm;
     b->form = h0->form;
     b->mem = members;
-    b->lz = DL_DEFAULT_LZ;
+    b->lz = 0;
     b->bps = 2;
     b->use_graph = 1;
     b->persistent = 0;
@@ -1463,7 +1597,7 @@ int batch_set_option(void* p, const char* key, long long v) {
 
 int batch_get_option(void* p, const char* key, long long* v) {
     BatchImpl* b = (BatchImpl*)p;
-    if (strcmp(key, "lz") == 0) *v = b->lz;
+    if (strcmp(key, "lz") == 0) *v = batch_lz(b);
     else if (strcmp(key, "blocks_per_sm") == 0) *v = b->bps;
     else if (strcmp(key, "graph") == 0) *v = b->use_graph;
     else if (strcmp(key, "persistent") == 0) *v = b->persistent;
@@ -1493,7 +1627,7 @@ static int batch_build(BatchImpl* b) {
     }
     for (int m = 0; m < nm; ++m) {
         dl_handle* h = b->mem[m];
-        h->lz = min(b->lz, h->nz);
+        h->lz = min(batch_lz(b), h->nz);
         for (int k = 0; k < 2; ++k) {
             if (b->push) {
                 push_args_at(h, k, b->h_ptable + ((size_t)k * nm + m) * psz);  // the projection is in the push body
@@ -1605,10 +1739,11 @@ static int batch_step_concurrent(BatchImpl* b, int nsteps) {
             DL_CUDA(h0, cudaStreamWaitEvent(b->workers[m % nw], b->fork, 0));
         }
     int rc = DL_OK;
+    const int lz = batch_lz(b);
     for (int s = 0; s < nsteps && rc == DL_OK; ++s)
         for (int m = 0; m < nm && rc == DL_OK; ++m) {
             dl_handle* h = b->mem[m];
-            h->lz = std::min(b->lz, h->nz);
+            h->lz = std::min(lz, h->nz);
             cudaStream_t own = h->stream;
             h->stream = b->workers[m % nw];
             rc = fast_step(h);

@@ -1039,6 +1039,7 @@ static void push_args(dl_handle* h, PushArgs& pa, bool settle) {
     a.fh = h->fsp.d_fh[h->fsp.par];
     a.fh_next = h->fsp.d_fh[1 - h->fsp.par];
     a.step = settle ? h->step : h->step + 1;
+    if (settle) a.lz = settle_lz(h);
     pa.pending = h->pushed ? 1 : 0;
     pa.walls_load = (h->pushed && h->P.walls) ? 1 : 0;
     // the load completes the streaming of step h->step

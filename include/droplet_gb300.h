@@ -294,7 +294,8 @@ int dl_profile_read(dl_handle* h, dl_profile_stats* out);
 
 /* Launch-shape knobs of the fused kernel (no reference counterpart: the
  * reference fixes its loop structure at compile time). key "lz": z planes
- * marched by one block (1..nz); "lz" = 0 restores the default. "prefetch" 0|1:
+ * marched by one block (1..nz); "lz" = 0, the default, chooses it from the
+ * domain's size and the GPU's SMs (read back: the value in use). "prefetch" 0|1:
  * bulk L2 prefetch of the next plane's pulled rows. "pipeline" 0|1 (single
  * phase): the next plane's pulls held in registers. "projection" 0|1 (band
  * forcing, default 1): the projection of the new u on the band modes done by
@@ -398,7 +399,8 @@ int dl_batch_set_stream(dl_batch* b, void* cuda_stream);
 int dl_batch_step(dl_batch* b, int nsteps);
 
 /* Knobs: "persistent" 0|1 (the mode above, default 0); "lz" z planes per
- * block or work item (default 32, at most a member's nz); "blocks_per_sm"
+ * block or work item (at most a member's nz; until it is set, chosen from the
+ * members' sizes); "blocks_per_sm"
  * persistent blocks per SM (1 or 2); "graph" 1 = replay step pairs of the
  * persistent launch from a CUDA graph. */
 int dl_batch_set_option(dl_batch* b, const char* key, int64_t value);
