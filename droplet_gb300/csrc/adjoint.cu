@@ -70,17 +70,46 @@ constexpr int ADJ_AUX = 22;  // aux rows: 9, LES dL/dG (9 .. 17), per-site wg (1
 
 constexpr int ADJ_NREP = 64;  // copies of the gradient accumulators (spreads the atomics)
 
-__device__ __forceinline__ int pmodi(int v, int n) {
-    v %= n;
-    return v < 0 ? v + n : v;
-}
 __device__ __forceinline__ constexpr float EW(int i) { return i == 0 ? 2.0f / 9.0f : (i <= 6 ? 1.0f / 9.0f : 1.0f / 72.0f); }
 __device__ __forceinline__ constexpr float FW(int i) { return i == 0 ? -7.0f / 3.0f : (i <= 6 ? 1.0f / 3.0f : 1.0f / 24.0f); }
 __device__ __forceinline__ constexpr float HW(int i) { return i == 0 ? 1.f : 0.f; }
 __device__ __forceinline__ constexpr float C2(int i) { return i == 0 ? 0.f : (i <= 6 ? 1.f : 3.f); }
 
-__device__ __forceinline__ unsigned nbr(const AdjArgs& a, int x, int y, int z, int dx, int dy, int dz) {
-    return (unsigned)pmodi(x + dx, a.nx) + (unsigned)a.nx * ((unsigned)pmodi(y + dy, a.ny) + (unsigned)a.ny * (unsigned)pmodi(z + dz, a.nz));
+// a site's coordinates and the wrapped offsets of the columns, rows and planes
+// around it: a neighbour's index is three additions (as three remainders of
+// x + dx, y + dy, z + dz it was a tenth of adj_local's and adj_stencil's time:
+// 91 -> 83 and 102 -> 97 us at 96^3)
+struct Near {
+    unsigned xo[3], yo[3], zo[3];
+    __device__ __forceinline__ Near(const AdjArgs& a, unsigned s) {
+        const unsigned nx = (unsigned)a.nx, ny = (unsigned)a.ny;
+        const unsigned row = s / nx;
+        const int x = (int)(s - row * nx), z = (int)(row / ny), y = (int)(row - (unsigned)z * ny);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            xo[d] = (unsigned)wrapi(x - 1 + d, a.nx);
+            yo[d] = nx * (unsigned)wrapi(y - 1 + d, a.ny);
+            zo[d] = nx * ny * (unsigned)wrapi(z - 1 + d, a.nz);
+        }
+    }
+    // x + c_i, x - c_i
+    __device__ __forceinline__ unsigned to(int i) const { return xo[1 + cx(i)] + yo[1 + cy(i)] + zo[1 + cz(i)]; }
+    __device__ __forceinline__ unsigned from(int i) const { return xo[1 - cx(i)] + yo[1 - cy(i)] + zo[1 - cz(i)]; }
+};
+
+// s + c v, c = -1, 0, 1
+__device__ __forceinline__ void addc(float& s, int c, float v) {
+    if (c > 0) s += v;
+    else if (c < 0) s -= v;
+}
+// c_i . (p, q, r)
+__device__ __forceinline__ float dotc(int i, float p, float q, float r) {
+    float s = 0.f;
+    bool any = false;
+    if (cx(i) != 0) { s = cx(i) > 0 ? p : -p; any = true; }
+    if (cy(i) != 0) { const float t = cy(i) > 0 ? q : -q; s = any ? s + t : t; any = true; }
+    if (cz(i) != 0) { const float t = cz(i) > 0 ? r : -r; s = any ? s + t : t; }
+    return s;
 }
 
 template <int NV>
@@ -100,6 +129,25 @@ __device__ __forceinline__ void block_add(double (&v)[NV], double* out) {
         for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += sh[threadIdx.x][w];
         atomicAdd(out + threadIdx.x, s);
     }
+}
+
+// the same for three FP32 values per thread (256 threads): a warp per value adds
+// its 256 in FP64, eight to a lane and then across lanes, 39 FP64 instructions
+// a block instead of 120 (every warp reducing in FP64 kept that pipe busy for a
+// third of adj_local's time)
+__device__ __forceinline__ void block_add3(const float (&v)[3], double* out) {
+    __shared__ float sh[3][256];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) sh[k][threadIdx.x] = v[k];
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp >= 3) return;
+    double s = (double)sh[warp][lane];
+#pragma unroll
+    for (int j = 1; j < 8; ++j) s += (double)sh[warp][lane + 32 * j];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) atomicAdd(out + warp, s);
 }
 
 // reflected pairs at the walls (reference i = 4,8,9,10,15 <- 7,12,13,14,11 at
@@ -135,13 +183,13 @@ __global__ void __launch_bounds__(256) adj_local(AdjArgs a) {
     const bool active = s0 < (long long)a.N;
     const unsigned s = active ? (unsigned)s0 : 0u;
     const unsigned N = a.N;
-    const int x = (int)(s % a.nx), y = (int)((s / a.nx) % a.ny), z = (int)(s / ((unsigned)a.nx * a.ny));
+    const Near w(a, s);
     const float* mac = a.mac;
-    const float dphi = mac[s], u1 = mac[N + s], u2 = mac[2 * N + s], u3 = mac[3 * N + s];
+    const float dphi = __ldg(mac + s), u1 = __ldg(mac + N + s), u2 = __ldg(mac + 2 * N + s), u3 = __ldg(mac + 3 * N + s);
     const float phi = a.phi1 + dphi;
     float v[Q];
 #pragma unroll
-    for (int i = 1; i < Q; ++i) v[i] = mac[nbr(a, x, y, z, cx(i), cy(i), cz(i))];
+    for (int i = 1; i < Q; ++i) v[i] = __ldg(mac + w.to(i));
     float lap = -14.f * dphi;
 #pragma unroll
     for (int i = 1; i < Q; ++i) lap += v[i];
@@ -149,9 +197,9 @@ __global__ void __launch_bounds__(256) adj_local(AdjArgs a) {
     float gr[3] = {0.f, 0.f, 0.f};
 #pragma unroll
     for (int i = 1; i < Q; ++i) {
-        gr[0] += cx(i) * v[i];
-        gr[1] += cy(i) * v[i];
-        gr[2] += cz(i) * v[i];
+        addc(gr[0], cx(i), v[i]);
+        addc(gr[1], cy(i), v[i]);
+        addc(gr[2], cz(i), v[i]);
     }
     gr[0] *= a.inv_grad;
     gr[1] *= a.inv_grad;
@@ -171,13 +219,13 @@ __global__ void __launch_bounds__(256) adj_local(AdjArgs a) {
     if (les) {
 #pragma unroll
         for (int k = 1; k < Q; ++k) {
-            const unsigned m = nbr(a, x, y, z, cx(k), cy(k), cz(k));
-            const float uk[3] = {mac[N + m], mac[2 * N + m], mac[3 * N + m]};
+            const unsigned m = w.to(k);
+            const float uk[3] = {__ldg(mac + N + m), __ldg(mac + 2 * N + m), __ldg(mac + 3 * N + m)};
 #pragma unroll
             for (int al = 0; al < 3; ++al) {
-                if (cx(k)) G[al][0] += cx(k) * uk[al];
-                if (cy(k)) G[al][1] += cy(k) * uk[al];
-                if (cz(k)) G[al][2] += cz(k) * uk[al];
+                addc(G[al][0], cx(k), uk[al]);
+                addc(G[al][1], cy(k), uk[al]);
+                addc(G[al][2], cz(k), uk[al]);
             }
         }
         float acc = 0.f;
@@ -205,30 +253,32 @@ __global__ void __launch_bounds__(256) adj_local(AdjArgs a) {
     // per-site sums in FP32 (15 terms); FP64 from the block sums on (GB300's FP64 rate is low)
     float dkf = 0.f, dkg = 0.f, domf = 0.f;
     const float wf = a.stream ? a.omf : 1.f, wg = a.stream ? wgs : 1.f;
-    const float dp = mac[4 * N + s];
+    const float dp = __ldg(mac + 4 * N + s);
     const float usq = u1 * u1 + u2 * u2 + u3 * u3;
 #pragma unroll
     for (int i = 0; i < Q; ++i) {
-        const unsigned src = a.stream ? nbr(a, x, y, z, cx(i), cy(i), cz(i)) : s;
-        const float ai = a.lin[(size_t)i * N + src];
-        const float bi = a.lin[(size_t)(Q + i) * N + src];
+        const unsigned src = a.stream ? w.to(i) : s;
+        const float ai = __ldg(a.lin + (size_t)i * N + src);
+        const float bi = __ldg(a.lin + (size_t)(Q + i) * N + src);
         const float Lf = wf * ai, Lg = wg * bi;
+        // (as sums of products by c, zeros included: the compiler's contractions, and with them
+        // the bits of the gradients, depend on this form)
         const float cu = cx(i) * u1 + cy(i) * u2 + cz(i) * u3;
         const float cg = cx(i) * gr[0] + cy(i) * gr[1] + cz(i) * gr[2];
         const float cGc = 4.5f * cg * cg - 1.5f * C2(i) * gsq;
         const float E = EW(i);
         if (a.stream) {
             const float dfeq = HW(i) * dphi + FW(i) * dA + E * (3.f * phi * cu + a.kf * cGc);
-            domf += ai * (dfeq - a.st[(size_t)i * N + s]);
+            domf += ai * (dfeq - __ldg(a.st + (size_t)i * N + s));
         }
         if (SPEC && a.stream) {
-            lF[0] += 3.f * E * cx(i) * bi;
-            lF[1] += 3.f * E * cy(i) * bi;
-            lF[2] += 3.f * E * cz(i) * bi;
+            if (cx(i)) lF[0] += 3.f * E * cx(i) * bi;
+            if (cy(i)) lF[1] += 3.f * E * cy(i) * bi;
+            if (cz(i)) lF[2] += 3.f * E * cz(i) * bi;
         }
         if (pw) {  // geq_i - g_i in deviations (the bulk E_i cancels)
             const float dgeq = E * (3.f * dp + 3.f * cu + 4.5f * cu * cu - 1.5f * usq + a.kg * cGc);
-            lw += bi * (dgeq - a.gst[(size_t)i * N + s]);
+            lw += bi * (dgeq - __ldg(a.gst + (size_t)i * N + s));
         }
         lphi += Lf * (HW(i) + 3.f * E * cu);
         lA += Lf * FW(i);
@@ -287,8 +337,8 @@ __global__ void __launch_bounds__(256) adj_local(AdjArgs a) {
     } else {
         dkf = dkg = domf = 0.f;
     }
-    double gv[3] = {(double)dkf, (double)dkg, (double)domf};
-    block_add<3>(gv, a.grads + 4 * (blockIdx.x % ADJ_NREP));
+    const float gv[3] = {dkf, dkg, domf};
+    block_add3(gv, a.grads + 4 * (blockIdx.x % ADJ_NREP));
 }
 
 // lphi(x) = lphi_loc(x) - 14 llap(x)/5 + sum_k [llap(x - c_k)/5 + c_k . lgrad(x - c_k)/10],
@@ -299,16 +349,27 @@ __global__ void __launch_bounds__(256) adj_stencil(AdjArgs a, float* phi_out) {
     const long long s0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (s0 >= (long long)a.N) return;
     const unsigned s = (unsigned)s0, N = a.N;
-    const int x = (int)(s % a.nx), y = (int)((s / a.nx) % a.ny), z = (int)(s / ((unsigned)a.nx * a.ny));
-    float lphi = a.aux[s] - 14.f * a.inv_lap * a.aux[N + s];
+    const Near w(a, s);
+    // the streamed part's loads first: all of a site's are in flight together
+    // (as plain loads between the stores, which might alias them, they came one
+    // direction after another: 97 us at 96^3, now 39.5)
+    float lf[Q], lg[Q];
+#pragma unroll
+    for (int i = 0; i < Q; ++i) {
+        const unsigned src = a.stream ? w.to(i) : s;
+        lf[i] = __ldg(a.lin + (size_t)i * N + src);
+        lg[i] = __ldg(a.lin + (size_t)(Q + i) * N + src);
+    }
+    float lphi = __ldg(a.aux + s) - 14.f * a.inv_lap * __ldg(a.aux + N + s);
 #pragma unroll
     for (int k = 1; k < Q; ++k) {
-        const unsigned m = nbr(a, x, y, z, -cx(k), -cy(k), -cz(k));
-        lphi += a.inv_lap * a.aux[N + m] +
-                a.inv_grad * (cx(k) * a.aux[2 * N + m] + cy(k) * a.aux[3 * N + m] + cz(k) * a.aux[4 * N + m]);
+        const unsigned m = w.from(k);
+        const float gx = cx(k) ? __ldg(a.aux + 2 * N + m) : 0.f, gy = cy(k) ? __ldg(a.aux + 3 * N + m) : 0.f;
+        const float gz = cz(k) ? __ldg(a.aux + 4 * N + m) : 0.f;
+        lphi += a.inv_lap * __ldg(a.aux + N + m) + a.inv_grad * dotc(k, gx, gy, gz);
     }
-    const float lp = a.aux[5 * N + s] * (1.f / 3.f);
-    float lu1 = a.aux[6 * N + s], lu2 = a.aux[7 * N + s], lu3 = a.aux[8 * N + s];
+    const float lp = __ldg(a.aux + 5 * N + s) * (1.f / 3.f);
+    float lu1 = __ldg(a.aux + 6 * N + s), lu2 = __ldg(a.aux + 7 * N + s), lu3 = __ldg(a.aux + 8 * N + s);
     float wg = a.stream ? a.omg : 1.f;
     if (LES && a.stream) {
         // transpose of G_ab(y) = inv_grad sum_k c_kb u_a(y + c_k): u_a(x) receives
@@ -316,13 +377,13 @@ __global__ void __launch_bounds__(256) adj_stencil(AdjArgs a, float* phi_out) {
         float t[3] = {0.f, 0.f, 0.f};
 #pragma unroll
         for (int k = 1; k < Q; ++k) {
-            const unsigned m = nbr(a, x, y, z, -cx(k), -cy(k), -cz(k));
+            const unsigned m = w.from(k);
 #pragma unroll
             for (int al = 0; al < 3; ++al) {
                 float v = 0.f;
-                if (cx(k)) v += cx(k) * a.aux[(size_t)(9 + al) * N + m];
-                if (cy(k)) v += cy(k) * a.aux[(size_t)(9 + al + 3) * N + m];
-                if (cz(k)) v += cz(k) * a.aux[(size_t)(9 + al + 6) * N + m];
+                if (cx(k)) addc(v, cx(k), __ldg(a.aux + (size_t)(9 + al) * N + m));
+                if (cy(k)) addc(v, cy(k), __ldg(a.aux + (size_t)(9 + al + 3) * N + m));
+                if (cz(k)) addc(v, cz(k), __ldg(a.aux + (size_t)(9 + al + 6) * N + m));
                 t[al] += v;
             }
         }
@@ -330,17 +391,14 @@ __global__ void __launch_bounds__(256) adj_stencil(AdjArgs a, float* phi_out) {
         lu2 += a.inv_grad * t[1];
         lu3 += a.inv_grad * t[2];
     }
-    if (PW && a.stream) wg = a.aux[(size_t)18 * N + s];
+    if (PW && a.stream) wg = __ldg(a.aux + (size_t)18 * N + s);
     if (phi_out) phi_out[s] = lphi;
-    // the streamed part (1 - w) of the collision, gathered here rather than
-    // stored by adj_local and read back
+    // the streamed part (1 - w) of the collision is gathered here rather than stored by adj_local and read back
     const float wf = a.stream ? a.omf : 1.f;
 #pragma unroll
     for (int i = 0; i < Q; ++i) {
-        const unsigned src = a.stream ? nbr(a, x, y, z, cx(i), cy(i), cz(i)) : s;
-        a.lout[(size_t)i * N + s] = (1.f - wf) * a.lin[(size_t)i * N + src] + lphi;
-        a.lout[(size_t)(Q + i) * N + s] =
-            (1.f - wg) * a.lin[(size_t)(Q + i) * N + src] + (lp + (cx(i) * lu1 + cy(i) * lu2 + cz(i) * lu3));
+        a.lout[(size_t)i * N + s] = (1.f - wf) * lf[i] + lphi;
+        a.lout[(size_t)(Q + i) * N + s] = (1.f - wg) * lg[i] + (lp + dotc(i, lu1, lu2, lu3));
     }
 }
 
