@@ -3,9 +3,11 @@
 // dissipation, droplet volume, pressure inside/outside, deformation moments).
 //
 // Two launches: per-block partial sums (one pass over the fields, per-thread
-// FP64 accumulators, warp-shuffle then shared-memory tree), then one warp
-// that adds the partials of every block in a fixed order with Neumaier
-// compensation, so the result is deterministic.
+// FP64 accumulators, warp-shuffle then shared-memory tree), then one
+// warp per quantity that adds the blocks' partials in a fixed order with
+// Neumaier compensation, so the result is deterministic. The FP64 pipe bounds
+// the first (280 -> 150 us at 128^3 FP32); the second waited for 304 loads and
+// additions one after another (126 -> 8 us).
 #include "dl_internal.cuh"
 #include "diag_site.cuh"
 
@@ -16,7 +18,7 @@ namespace dl {
 constexpr int NSUM = DIAG_NSUM;  // sums, then min, max
 constexpr int NPART = NSUM + 2;
 constexpr int RED_BLOCKS = 304;  // 2 x 152 SMs
-constexpr int RED_THREADS = 256;
+constexpr int RED_THREADS = DIAG_NT;
 
 struct RedArgs {
     DiagConsts k;
@@ -29,16 +31,26 @@ __global__ void __launch_bounds__(RED_THREADS) reduce_partials(const T* __restri
 #pragma unroll
     for (int k = 0; k < NSUM; ++k) acc[k] = 0.0;
     double vmin = INFINITY, vmax = -INFINITY;
-    diag_sites(mac, a.k, blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x, acc, vmin,
-               vmax);
+    __shared__ DiagRing<T> ring;
+    diag_sites(mac, a.k, ring, blockIdx.x, gridDim.x, acc, vmin, vmax);
     __shared__ double sh[RED_THREADS / 32][NPART];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // warp sums, transposed: each exchange halves the values a lane holds, and
+    // lane k ends with the sum of value k (31 FP64 additions instead of 120)
+    {
+        double v[32];
 #pragma unroll
-    for (int k = 0; k < NSUM; ++k) {
-        double v = acc[k];
+        for (int k = 0; k < 32; ++k) v[k] = k < NSUM ? acc[k < NSUM ? k : 0] : 0.0;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0) sh[warp][k] = v;
+        for (int h = 16; h >= 1; h >>= 1) {
+            const bool up = (lane & h) != 0;
+#pragma unroll
+            for (int j = 0; j < h; ++j) {
+                const double send = up ? v[j] : v[j + h], keep = up ? v[j + h] : v[j];
+                v[j] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+            }
+        }
+        if (lane < NSUM) sh[warp][lane] = v[0];
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -62,25 +74,46 @@ __global__ void __launch_bounds__(RED_THREADS) reduce_partials(const T* __restri
     }
 }
 
-__global__ void reduce_final(const double* __restrict__ part, int nblocks, double* __restrict__ out) {
-    const int k = threadIdx.x;
-    if (k >= NPART) return;
-    if (k == NSUM || k == NSUM + 1) {
-        double v = part[k];
-        for (int b = 1; b < nblocks; ++b) v = (k == NSUM) ? fmin(v, part[b * NPART + k]) : fmax(v, part[b * NPART + k]);
-        out[k] = v;
-        return;
+__device__ __forceinline__ void neumaier_add(double& s, double& c, double v) {
+    const double t = s + v;
+    if (fabs(s) >= fabs(v)) c += (s - t) + v;
+    else c += (v - t) + s;
+    s = t;
+}
+
+// block k: quantity k (blocks of one warp, each on an SM of its own: the FP64
+// pipe of one SM would take all 26 in turn). A lane adds every 32nd partial, then
+// the lanes' sums and compensations are folded pairwise
+__global__ void __launch_bounds__(32) reduce_final(const double* __restrict__ part, int nblocks,
+                                                           double* __restrict__ out) {
+    const int k = blockIdx.x, lane = threadIdx.x;
+    const bool is_min = k == NSUM, is_max = k == NSUM + 1;
+    double s = is_min ? INFINITY : is_max ? -INFINITY : 0.0, c = 0.0;
+    constexpr int U = (RED_BLOCKS + 31) / 32;
+    double v[U];
+#pragma unroll
+    for (int j = 0; j < U; ++j) {
+        const int b = lane + 32 * j;
+        v[j] = part[(b < nblocks ? b : 0) * NPART + k];
     }
-    // Neumaier-compensated sum in block order
-    double s = 0.0, c = 0.0;
-    for (int b = 0; b < nblocks; ++b) {
-        const double v = part[b * NPART + k];
-        const double t = s + v;
-        if (fabs(s) >= fabs(v)) c += (s - t) + v;
-        else c += (v - t) + s;
-        s = t;
+#pragma unroll
+    for (int j = 0; j < U; ++j) {
+        if (lane + 32 * j >= nblocks) continue;
+        if (is_min) s = fmin(s, v[j]);
+        else if (is_max) s = fmax(s, v[j]);
+        else neumaier_add(s, c, v[j]);
     }
-    out[k] = s + c;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double s2 = __shfl_down_sync(0xffffffffu, s, o), c2 = __shfl_down_sync(0xffffffffu, c, o);
+        if (is_min) s = fmin(s, s2);
+        else if (is_max) s = fmax(s, s2);
+        else {
+            neumaier_add(s, c, s2);
+            c += c2;
+        }
+    }
+    if (lane == 0) out[k] = (is_min || is_max) ? s : s + c;
 }
 
 // the per-site constants of the diagnostics for handle h (shared with dl_reduce_static)
@@ -106,9 +139,10 @@ static int reduce_any(dl_handle* h, const T* d_mac, double phi_off, double p_off
     RedArgs a;
     memset(&a, 0, sizeof(a));
     diag_consts(h, phi_off, p_off, a.k);
+    a.k.chunk = diag_chunk(h->nx, h->ny, h->nz, RED_BLOCKS);
     a.part = h->d_diag;
     DL_LAUNCH(h, false, reduce_partials<T><<<RED_BLOCKS, RED_THREADS, 0, h->stream>>>(d_mac, a));
-    DL_LAUNCH(h, false, reduce_final<<<1, 32, 0, h->stream>>>(h->d_diag, RED_BLOCKS, h->d_diag + RED_BLOCKS * NPART));
+    DL_LAUNCH(h, false, reduce_final<<<NPART, 32, 0, h->stream>>>(h->d_diag, RED_BLOCKS, h->d_diag + RED_BLOCKS * NPART));
     DL_CUDA(h, cudaGetLastError());
     double r[NPART];
     DL_CUDA(h, cudaMemcpyAsync(r, h->d_diag + RED_BLOCKS * NPART, sizeof(r), cudaMemcpyDeviceToHost, h->stream));

@@ -60,6 +60,8 @@ __device__ __forceinline__ void rs_add(double& s, double& c, double v) {
     s = t;
 }
 
+static_assert(RS_THREADS == DIAG_NT, "the blocks of diag_sites");
+
 template <typename T>
 __global__ void __launch_bounds__(RS_THREADS) reduce_static_kernel(const T* __restrict__ mac, const RsArgs a,
                                                                    double* __restrict__ scratch) {
@@ -71,8 +73,8 @@ __global__ void __launch_bounds__(RS_THREADS) reduce_static_kernel(const T* __re
 #pragma unroll
     for (int k = 0; k < RS_NSUM; ++k) acc[k] = 0.0;
     double vmin = INFINITY, vmax = -INFINITY;
-    diag_sites(mac, a.k, blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x, acc, vmin,
-               vmax);
+    __shared__ DiagRing<T> ring;
+    diag_sites(mac, a.k, ring, blockIdx.x, gridDim.x, acc, vmin, vmax);
 
     // block partials: warp shuffles, then one row per warp in shared memory
     __shared__ double sh[RS_THREADS / 32][RS_NPART];
@@ -217,6 +219,7 @@ static int reduce_static_any(dl_handle* h, const T* d_mac, double phi_off, doubl
     RsArgs a;
     memset(&a, 0, sizeof(a));
     diag_consts(h, phi_off, p_off, a.k);
+    a.k.chunk = diag_chunk(h->nx, h->ny, h->nz, nblocks);
     // the arrival counter starts at zero whatever an earlier launch left
     DL_CUDA(h, cudaMemsetAsync(scratch + (size_t)RS_MAX_BLOCKS * RS_NPART + RS_NPART, 0, sizeof(unsigned long long),
                                h->stream));
