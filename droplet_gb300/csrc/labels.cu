@@ -7,11 +7,17 @@
 // join is made; the connectivity is selectable and includes the reference's
 // neighbour set made symmetric (faces plus the xz and yz edges).
 //
-// Union-find on the device: parent[s] = s for a foreground site; every site
-// unites with the forward half of its neighbour set, linking the larger root
-// under the smaller one with atomicCAS (parents only decrease, so every chain
-// is finite); then each site points at its root, roots count their sites,
-// and roots get compact ids.
+// Union-find on the device. A foreground site starts under the first site of
+// its run within its warp's 32 consecutive sites of the row (no atomics); then
+// sites unite with the forward half of their neighbour set, linking the larger
+// root under the smaller one with atomicCAS (parents only decrease, so every
+// chain is finite) and halving the paths they walk; a pair whose left
+// neighbours are a pair of the same two runs is left to them. Then each site
+// points at its root, roots count their sites (one atomic per root and warp),
+// get compact ids and, by volume on the host, their rank, which the last pass
+// writes as the label. Measured on 256^3 with 24 droplets of radius 8 to 24 (us,
+// before with a union per pair and no path halving / now): union 1386 / 112, init
+// 51 / 50, count 103 / 47, labels 44 and a host pass of 5.5 ms / 44.
 #include "dl_internal.cuh"
 #include "dl_device.cuh"
 
@@ -44,35 +50,59 @@ __device__ __forceinline__ bool fg(const LabelArgs& a, int s) {
 
 constexpr int LBL_MAXIT = 1 << 24;
 
+// the root of x; a walked site is moved up to its grandparent (a plain store: any
+// value written is an ancestor, so a racing reader only takes a longer way)
 __device__ __forceinline__ int find_root(const LabelArgs& a, int x) {
+    int p = __ldcg(a.parent + x);
     for (int it = 0; it < LBL_MAXIT; ++it) {
-        const int p = __ldcg(a.parent + x);
         if (p == x) return x;
+        const int g = __ldcg(a.parent + p);
+        if (g == p) return p;
+        __stcg(a.parent + x, g);
         x = p;
+        p = g;
     }
     atomicExch(a.err, 1);
     return x;
 }
 
-__global__ void lbl_init(LabelArgs a) {
+__global__ void __launch_bounds__(256) lbl_init(LabelArgs a) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool in = s < a.N && fg(a, s);
+    const unsigned mask = __ballot_sync(0xffffffffu, in);
     if (s >= a.N) return;
-    a.parent[s] = fg(a, s) ? s : -1;
-    a.count[s] = 0;
+    const int lane = threadIdx.x & 31;
+    int start = -1;
+    if (in) {
+        // first site of the run: after the nearest background site below, within the warp and the row
+        const unsigned below = ~mask & ((1u << lane) - 1u);
+        const int first = below ? 32 - __clz(below) : 0;
+        start = s - min(lane - first, s % a.nx);
+        if (start == s) a.count[s] = 0;  // a root is always a run's first site
+    }
+    a.parent[s] = start;
 }
 
-__global__ void lbl_union(LabelArgs a) {
+__global__ void __launch_bounds__(256) lbl_union(LabelArgs a) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= a.N || __ldcg(a.parent + s) < 0) return;
-    const int x = s % a.nx, y = (s / a.nx) % a.ny, z = s / (a.nx * a.ny);
+    const int row = s / a.nx, x = s - row * a.nx, z = row / a.ny, y = row - z * a.ny;
+    const bool left = x > 0 && __ldcg(a.parent + s - 1) >= 0;  // the site before is of the same run
     for (int d = 0; d < a.ndir; ++d) {
         const int3 o = a.dirs[d];
         int xx = x + o.x, yy = y + o.y, zz = z + o.z;
+        const bool wrapped = xx < 0 || xx >= a.nx;
         xx = xx < 0 ? xx + a.nx : (xx >= a.nx ? xx - a.nx : xx);
         yy = yy < 0 ? yy + a.ny : (yy >= a.ny ? yy - a.ny : yy);
         zz = zz < 0 ? zz + a.nz : (zz >= a.nz ? zz - a.nz : zz);
         const int t = xx + a.nx * (yy + a.ny * zz);
         if (__ldcg(a.parent + t) < 0) continue;
+        if (o.y == 0 && o.z == 0) {
+            // along the row: lbl_init joined all but the ends of warps (runs start anew there) and of the row
+            if (!wrapped && (t & 31) != 0) continue;
+        } else if (left && !wrapped && xx > 0 && (x - 1 + o.x >= 0) && __ldcg(a.parent + t - 1) >= 0) {
+            continue;  // s - 1 and t - 1 unite the two runs
+        }
         int u = s, v = t;
         for (int it = 0; it < LBL_MAXIT; ++it) {
             u = find_root(a, u);
@@ -91,12 +121,15 @@ __global__ void lbl_union(LabelArgs a) {
     }
 }
 
-__global__ void lbl_compress_count(LabelArgs a) {
+__global__ void __launch_bounds__(256) lbl_compress_count(LabelArgs a) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= a.N || a.parent[s] < 0) return;
+    const bool in = s < a.N && a.parent[s] >= 0;
+    const unsigned who = __ballot_sync(0xffffffffu, in);
+    if (!in) return;
     const int r = find_root(a, s);
     a.parent[s] = r;
-    atomicAdd(a.count + r, 1);
+    const unsigned same = __match_any_sync(who, r);
+    if ((threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(a.count + r, __popc(same));
 }
 
 __global__ void lbl_compact(LabelArgs a) {
@@ -109,11 +142,12 @@ __global__ void lbl_compact(LabelArgs a) {
     }
 }
 
-__global__ void lbl_final(LabelArgs a, int* out) {
+// labels: the rank of the site's root, rank[id - 1] = 1 for the largest
+__global__ void lbl_final(LabelArgs a, const int* __restrict__ rank, int* __restrict__ out) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= a.N) return;
     const int r = a.parent[s];
-    out[s] = r < 0 ? 0 : a.ids[r];
+    out[s] = r < 0 ? 0 : rank[a.ids[r] - 1];
 }
 
 static void directions(int conn, LabelArgs& a) {
@@ -181,12 +215,13 @@ int label_droplets(dl_handle* h, int conn, int* labels_host, long long* ndrops, 
     *ndrops = n;
     for (long long i = 0; i < n && i < maxv; ++i) volumes[i] = (double)vols[order[i]];
     if (labels_host) {
-        DL_LAUNCH(h, false, (lbl_final<<<nb, 256, 0, h->stream>>>(a, a.count)));
+        // ranks over the volumes, which have been read; labels over the counts
+        for (int i = 0; i < n; ++i) vols[order[i]] = i + 1;
+        if (n) DL_CUDA(h, cudaMemcpyAsync(a.vols, vols.data(), sizeof(int) * n, cudaMemcpyHostToDevice, h->stream));
+        DL_LAUNCH(h, false, (lbl_final<<<nb, 256, 0, h->stream>>>(a, a.vols, a.count)));
+        DL_CUDA(h, cudaGetLastError());
         DL_CUDA(h, cudaMemcpyAsync(labels_host, a.count, sizeof(int) * (size_t)N, cudaMemcpyDeviceToHost, h->stream));
         DL_CUDA(h, cudaStreamSynchronize(h->stream));
-        std::vector<int> rank((size_t)n + 1, 0);
-        for (int i = 0; i < n; ++i) rank[order[i] + 1] = i + 1;
-        for (int s = 0; s < N; ++s) labels_host[s] = rank[labels_host[s]];
     }
     return DL_OK;
 }
