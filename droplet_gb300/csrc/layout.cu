@@ -7,32 +7,45 @@
 
 namespace dl {
 
-__global__ void soa_to_aos_kernel(const double* __restrict__ soa, double* __restrict__ aos, long long N) {
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= (long long)Q * N) return;
-    const long long s = t / Q;
-    const int i = (int)(t - s * Q);
-    aos[t] = soa[i * N + s];
+// a block's sites through shared memory: both sides are read and written as runs
+// (the strided side alone touched eight times its sectors)
+constexpr int LAYOUT_NT = 128;
+
+__global__ void __launch_bounds__(LAYOUT_NT) soa_to_aos_kernel(const double* __restrict__ soa, double* __restrict__ aos,
+                                                               long long N) {
+    __shared__ double buf[LAYOUT_NT * Q];
+    const long long s0 = blockIdx.x * (long long)LAYOUT_NT, s = s0 + threadIdx.x;
+    if (s < N) {
+#pragma unroll
+        for (int i = 0; i < Q; ++i) buf[threadIdx.x * Q + i] = __ldg(soa + i * N + s);
+    }
+    __syncthreads();
+    const int n = (int)min((long long)LAYOUT_NT, N - s0) * Q;
+    for (int t = threadIdx.x; t < n; t += LAYOUT_NT) aos[s0 * Q + t] = buf[t];
 }
 
-__global__ void aos_to_soa_kernel(const double* __restrict__ aos, double* __restrict__ soa, long long N) {
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= (long long)Q * N) return;
-    const int i = (int)(t / N);
-    const long long s = t - i * N;
-    soa[t] = aos[s * Q + i];
+__global__ void __launch_bounds__(LAYOUT_NT) aos_to_soa_kernel(const double* __restrict__ aos, double* __restrict__ soa,
+                                                               long long N) {
+    __shared__ double buf[LAYOUT_NT * Q];
+    const long long s0 = blockIdx.x * (long long)LAYOUT_NT, s = s0 + threadIdx.x;
+    const int n = (int)min((long long)LAYOUT_NT, N - s0) * Q;
+    for (int t = threadIdx.x; t < n; t += LAYOUT_NT) buf[t] = __ldg(aos + s0 * Q + t);
+    __syncthreads();
+    if (s >= N) return;
+#pragma unroll
+    for (int i = 0; i < Q; ++i) soa[i * N + s] = buf[threadIdx.x * Q + i];
 }
+
+static unsigned layout_blocks(const dl_handle* h) { return (unsigned)((h->N + LAYOUT_NT - 1) / LAYOUT_NT); }
 
 int soa_to_aos(dl_handle* h, const double* d_soa, double* d_aos) {
-    const long long n = (long long)Q * h->N;
-    DL_LAUNCH(h, false, soa_to_aos_kernel<<<(unsigned)((n + 255) / 256), 256, 0, h->stream>>>(d_soa, d_aos, (long long)h->N));
+    DL_LAUNCH(h, false, soa_to_aos_kernel<<<layout_blocks(h), LAYOUT_NT, 0, h->stream>>>(d_soa, d_aos, (long long)h->N));
     DL_CUDA(h, cudaGetLastError());
     return DL_OK;
 }
 
 int aos_to_soa(dl_handle* h, const double* d_aos, double* d_soa) {
-    const long long n = (long long)Q * h->N;
-    DL_LAUNCH(h, false, aos_to_soa_kernel<<<(unsigned)((n + 255) / 256), 256, 0, h->stream>>>(d_aos, d_soa, (long long)h->N));
+    DL_LAUNCH(h, false, aos_to_soa_kernel<<<layout_blocks(h), LAYOUT_NT, 0, h->stream>>>(d_aos, d_soa, (long long)h->N));
     DL_CUDA(h, cudaGetLastError());
     return DL_OK;
 }
