@@ -395,6 +395,7 @@ int dl_set_option(dl_handle* h, const char* key, int64_t value) {
     if (strcmp(key, "push") == 0) {
         if (value < 0 || value > 1) return set_error(h, DL_ERR_ARG, "push must be 0 or 1");
         h->push = (int)value;
+        memset(h->lz_auto, 0, sizeof(h->lz_auto));  // the choice depends on it
         return DL_OK;
     }
     if (strcmp(key, "stage") == 0) {
@@ -402,6 +403,7 @@ int dl_set_option(dl_handle* h, const char* key, int64_t value) {
         if (value == 2 && !push_tma_eligible(h))
             return set_error(h, DL_ERR_UNSUPPORTED, "stage 2 (tensor copies) needs nx a multiple of 32 and ny of 8");
         h->push_bulk = (int)value;
+        memset(h->lz_auto, 0, sizeof(h->lz_auto));
         return DL_OK;
     }
     if (strcmp(key, "wait_ns") == 0) {

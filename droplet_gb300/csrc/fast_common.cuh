@@ -549,6 +549,8 @@ __device__ __forceinline__ void spectral_block_done(const FastArgs& a, float* sc
 // host side shared by the pull (step_fast.cu) and push (step_push.cu) forms
 void fill_fast(dl_handle* h, FastArgs& a);
 int sm_count(dl_handle* h);
+bool chunked_projection(dl_handle* h);
+int launch_projection(dl_handle* h, const FastArgs& a);
 int force_fmode(const dl_handle* h);
 void advance(dl_handle* h, int n);
 void wall_terms(const dl_handle* h, long long step, float* bot, float* top);

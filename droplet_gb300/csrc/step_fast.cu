@@ -722,9 +722,10 @@ __global__ void __launch_bounds__(PROJ_NT, 4) sp_project_fast(const FastArgs a) 
 
 // the projection of the fused step as a launch of its own, over chunks of
 // BAND_CHUNK planes whatever the step's lz: the same sums in the same order as
-// a step whose blocks march BAND_CHUNK planes. FP16 storage turns any change of
-// rounding in the force into one FP16 quantum here and there, which spreads, so
-// its band sums must not depend on how the step is cut.
+// a step whose blocks march BAND_CHUNK planes, so that the two-phase results do
+// not depend on how the step is cut: FP16 storage turns any change of rounding in
+// the force into one FP16 quantum here and there, which spreads, and FP32
+// checkpoints after a few steps are otherwise 1e-9 apart.
 constexpr int BAND_CHUNK = 32;
 __global__ void __launch_bounds__(NT) project_chunks(const FastArgs a) {
     __shared__ __align__(16) float scr[PT_SCRATCH];
@@ -972,9 +973,7 @@ int sm_count(dl_handle* h) {
 // rest costs a lone block's time when nothing ran before it on its SM, but
 // 0.9 of a full block's otherwise (the waves do not end together). The
 // candidates split nz evenly. Measured (us per step, at the constant 32 that
-// this replaces / at the chosen lz): FP32 LES and band forcing 32^3 122 / 24
-// (lz 1), 64^3 122 / 42 (4), 96^3 135 / 88 (12), 128^3 188 / 188 (32), 256^3
-// 1315 / 1289 (37); shear droplet 32^3 61 / 10, 64^3 69 / 20; pull form 96^3
+// this replaces / at the chosen lz): shear droplet 32^3 61 / 10, 64^3 69 / 20; pull form 96^3
 // 166 / 92; FP16 96^3 162 / 100. Over 13 shapes and five step variants the
 // choice is within 5 % of the best of a sweep.
 static double march_cost(int lz, const dl_handle* h, int sms, double prol) {
@@ -1004,13 +1003,22 @@ static int march_planes(const dl_handle* h, int sms, double prol) {
 static int prologue_class(const dl_handle* h) { return force_fmode(h) != F_SPECTRAL ? 0 : h->single ? 2 : 1; }
 static const double PROLOGUE_PLANES[3] = {1.0, 2.5, 5.0};
 
-// FP16 storage with band forcing: another lz than BAND_CHUNK needs the
-// projection as a launch of its own (project_chunks), about CHUNK_LAUNCH planes'
-// time (it hides no latency behind a march); it pays on small domains
-// (us per step at lz 32 before / now: 32^3 127 / 32, 64^3 133 / 51, 96^3
-// 165 / 107, 256^3 1525 / 1485)
-constexpr double CHUNK_LAUNCH = 2.0;
-static bool band_fp16(const dl_handle* h) { return h->form == DL_FORM_FP16 && force_fmode(h) == F_SPECTRAL; }
+// The two-phase step with band forcing sums its projection in FP32 per chunk of
+// BAND_CHUNK planes; another lz needs the projection as a launch of its own
+// (project_chunks) to keep those sums: about two planes' time (it hides no
+// latency behind a march), and for the push form, which then stores u, an eighth
+// of the march. It pays on domains that lz = 32 cuts badly (us per step at lz 32
+// / at the choice; FP16 32^3 127 / 32, 64^3 133 / 51, 96^3 165 / 107, 256^3 1525 /
+// 1485; FP32 push 32^3 119 / 33, 64^3 122 / 52, 96^3 129 / 99, 160^3 342 / 335;
+// not on 256^3, 1210 / 1332).
+static double chunked_cost(const dl_handle* h, double march) {
+    return 2.0 + (h->form == DL_FORM_FP32 ? 1.12 : 1.0) * march;
+}
+static bool band_two_phase(const dl_handle* h) {
+    return force_fmode(h) == F_SPECTRAL && (!h->single || h->form == DL_FORM_FP16);
+}
+// step_push_u has no staged variants
+static bool has_chunked_step(const dl_handle* h) { return !(push_eligible(h) && h->push_bulk != 0); }
 
 int effective_lz(dl_handle* h) {
     if (h->lz > 0) return h->lz;
@@ -1020,7 +1028,8 @@ int effective_lz(dl_handle* h) {
         const double prol = PROLOGUE_PLANES[c];
         int lz = march_planes(h, sms, prol);
         const int chunk = std::min(h->nz, BAND_CHUNK);
-        if (band_fp16(h) && march_cost(chunk, h, sms, prol) <= march_cost(lz, h, sms, prol) + CHUNK_LAUNCH)
+        if (band_two_phase(h) &&
+            (!has_chunked_step(h) || march_cost(chunk, h, sms, prol) <= chunked_cost(h, march_cost(lz, h, sms, prol))))
             lz = chunk;
         h->lz_auto[c] = lz;
     }
@@ -1037,8 +1046,8 @@ int settle_lz(dl_handle* h) {
 }
 
 // the step's band projection is project_chunks instead of the fused step's own
-static bool chunked_projection(dl_handle* h) {
-    return band_fp16(h) && h->proj_in_step && h->lz == 0 && effective_lz(h) != std::min(h->nz, BAND_CHUNK);
+bool chunked_projection(dl_handle* h) {
+    return band_two_phase(h) && h->proj_in_step && h->lz == 0 && effective_lz(h) != std::min(h->nz, BAND_CHUNK);
 }
 
 void fill_fast(dl_handle* h, FastArgs& a) {
@@ -1258,7 +1267,7 @@ static const int PROJ_ROWS = 64;  // rows of the band projection per block (batc
 
 // band projection launch: four blocks on every SM (the register limit), one
 // wave; fewer blocks when there are fewer rows than warps
-static int launch_projection(dl_handle* h, const FastArgs& a) {
+int launch_projection(dl_handle* h, const FastArgs& a) {
     if (chunked_projection(h)) {
         const dim3 grid((a.nx + TX - 1) / TX, (a.ny + TY - 1) / TY, (a.nz + BAND_CHUNK - 1) / BAND_CHUNK);
         DL_LAUNCH(h, false, (project_chunks<<<grid, NT, 0, h->stream>>>(a)));
@@ -1504,7 +1513,7 @@ static int batch_lz(BatchImpl* b) {
     for (int m = 0; m < b->nm; ++m) nzmax = std::max(nzmax, b->mem[m]->nz);
     int best = BAND_CHUNK;
     double cost = INFINITY;
-    for (int k = (nzmax + 63) / 64; k <= nzmax && !band_fp16(b->mem[0]); ++k) {  // at most 64 planes
+    for (int k = (nzmax + 63) / 64; k <= nzmax && !band_two_phase(b->mem[0]); ++k) {  // at most 64 planes
         const int lz = (nzmax + k - 1) / k;
         double planes = 0.0;
         for (int m = 0; m < b->nm; ++m) {

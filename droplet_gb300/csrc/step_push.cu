@@ -51,7 +51,13 @@
 namespace dl {
 
 constexpr int PSL = 4;   // ring slots (moments and band force)
-constexpr int FENT = 4;  // band force entry: Fx, Fy, Fz, padding
+// band force entry Fx, Fy, Fz, three words without padding: with four (one 16-byte read per
+// diagonal direction instead of three 4-byte ones) the two-phase block takes 70 KB of shared
+// memory and two blocks leave 92 KB of L1; at 63 KB the SM's split leaves 124 KB to the
+// register spill (128^3 LES and band forcing 184 -> 175 us per step), and the 16-byte reads
+// took four passes anyway (single phase 256^3 595 -> 577)
+constexpr int FENT = 3;
+constexpr int FCOL = 4;  // float4 groups of a column's band-force coefficients (15 values)
 constexpr int NHALO = 2 * EX1 + 2 * TY;  // 84 positions of the one-cell ring
 static_assert(NHALO <= NT, "one halo site per thread at most");
 static_assert((PSL & (PSL - 1)) == 0, "ring slots by bit mask");
@@ -135,15 +141,18 @@ __host__ __device__ constexpr int pb_goff(bool sp) { return sp ? 0 : Q * NT; }
 // (rings and tables, then, stage 1 or 2, the staged plane at a 128-byte
 // offset, then, stage 2, its mbarrier and 128 bytes of room to move the plane
 // to a 128-byte boundary of the shared window, where tensor copies land)
-__host__ __device__ constexpr int push_rings_floats(bool spec, bool sp) {
+// (the band force of a march comes from a per-plane table, of a march without
+// stencils or a settle from the columns' coefficients: see fcolumns)
+__host__ __device__ constexpr int push_rings_floats(bool spec, bool sp, bool cols) {
     return (sp ? 0 : PSL * P1 * 4 + 2 * Q * NHALO) +
-           (spec ? PSL * P2 * FENT + 2 * (3 * SNK * EY2 * 2) + 3 * SNK * EY2 * 3 * 2 + SNK * EX2 * 2 +
-                       SNK * EY2 * 2 + SNK * EX1 * 2 + SNK * EY1 * 2
+           (spec ? PSL * P2 * FENT + SNK * EX1 * 2 + SNK * EY1 * 2 +
+                       (cols ? FCOL * P2 * 4
+                             : 2 * (3 * SNK * EY2 * 2) + 3 * SNK * EY2 * 3 * 2 + SNK * EX2 * 2 + SNK * EY2 * 2)
                  : 0);
 }
-__host__ __device__ constexpr int push_stage_offset(bool spec, bool sp) { return (push_rings_floats(spec, sp) + 31) / 32 * 32; }
-__host__ __device__ constexpr int push_smem_floats(bool spec, bool sp, int stage = 0) {
-    return stage == 0 ? push_rings_floats(spec, sp) : push_stage_offset(spec, sp) + pb_floats(sp) + (stage == 2 ? 36 : 0);
+__host__ __device__ constexpr int push_stage_offset(bool spec, bool sp) { return (push_rings_floats(spec, sp, sp) + 31) / 32 * 32; }
+__host__ __device__ constexpr int push_smem_floats(bool spec, bool sp, int stage = 0, bool settle = false) {
+    return stage == 0 ? push_rings_floats(spec, sp, sp || settle) : push_stage_offset(spec, sp) + pb_floats(sp) + (stage == 2 ? 36 : 0);
 }
 static_assert(PSL * P1 * 4 + PSL * P2 * FENT >= PT_SCRATCH, "projection scratch exceeds the rings");
 
@@ -455,23 +464,27 @@ __device__ __forceinline__ void push_minmax(const FastArgs& a, float bmin, float
 // registers after the collision: by each thread for its own site (4-byte
 // asynchronous copies, STG 1), or by one thread for the block (two tensor
 // copies completing on an mbarrier, STG 2; full tiles only)
-template <bool LES, int FMODE, bool SP, bool SETTLE, int STG = 0>
+template <bool LES, int FMODE, bool SP, bool SETTLE, int STG = 0, bool UOUT = false>
 __device__ __forceinline__ void push_body(const PushArgs& pa, float* smem, int bx, int by, int bz, unsigned nblk) {
     constexpr bool BULK = STG != 0;
     constexpr bool TMA = STG == 2;
     constexpr bool SPEC = FMODE == F_SPECTRAL;
     constexpr bool HALO = !SP && !SETTLE;  // the ring around the tile (stencils)
     constexpr bool NEEDG_HALO = LES;       // halo sites need u (strain) only with LES
+    constexpr bool COLS = SP || SETTLE;    // band force from the columns' coefficients (fcolumns)
     const FastArgs& a = pa.a;
     float4* s_mom = reinterpret_cast<float4*>(smem);              // [PSL][P1] (dphi, u1, u2, u3)
     float* s_h = smem + PSL * P1 * 4;                              // [2 Q][NHALO] halo sites' populations
     float* s_fr = smem + (SP ? 0 : PSL * P1 * 4 + 2 * Q * NHALO);  // [PSL][P2][FENT]
-    float2* s_C = reinterpret_cast<float2*>(s_fr + PSL * P2 * FENT);  // [2][3][SNK][EY2]
-    float2* s_D = s_C + 2 * 3 * SNK * EY2;                         // [3][SNK][EY2][3]
+    float2* s_tx1 = reinterpret_cast<float2*>(s_fr + PSL * P2 * FENT);  // [SNK][EX1] projection tables
+    float2* s_ty1 = s_tx1 + SNK * EX1;                             // [SNK][EY1]
+    float4* s_fc = reinterpret_cast<float4*>(s_ty1 + SNK * EY1);   // COLS: [FCOL][P2] columns' coefficients
+    // the tables of the per-plane synthesis; with COLS they are only used while the
+    // coefficients are made, in the force ring that they precede
+    float2* s_D = COLS ? reinterpret_cast<float2*>(s_fr) : s_ty1 + SNK * EY1;  // [3][SNK][EY2][3]
     float2* s_tx2 = s_D + 3 * SNK * EY2 * 3;                       // [SNK][EX2] (cos, -sin) kx x, x = x0-2+ex
     float2* s_ty2 = s_tx2 + SNK * EX2;                             // [SNK][EY2] e^{i ky y}, y = y0-2+ey
-    float2* s_tx1 = s_ty2 + SNK * EY2;                             // [SNK][EX1] projection tables
-    float2* s_ty1 = s_tx1 + SNK * EX1;                             // [SNK][EY1]
+    float2* s_C = s_ty2 + SNK * EY2;                               // [2][3][SNK][EY2] (not COLS)
     float* s_pb = smem + push_stage_offset(SPEC, SP);  // staged plane (BULK): [2 Q][NT], single phase [Q][NT]
     if (TMA) {  // at a 128-byte boundary of the shared window (the room is in the footprint)
         const unsigned off = (unsigned)__cvta_generic_to_shared(s_pb);
@@ -541,6 +554,7 @@ __device__ __forceinline__ void push_body(const PushArgs& pa, float* smem, int b
     };
     // C[c][kx][row] of plane zr into slot zr & 1
     auto ctable = [&](int zr) {
+        if (COLS) return;
         float2 ez1, ez2;
         ztw(zr, ez1, ez2);
         float2* C = s_C + (zr & 1) * (3 * SNK * EY2);
@@ -551,7 +565,7 @@ __device__ __forceinline__ void push_body(const PushArgs& pa, float* smem, int b
         }
     };
     // band force of plane zr at every position of the two-cell ring, from slot zr & 1 of C
-    auto fsynth = [&](int zr) {
+    auto fsynth_table = [&](int zr) {
         const float2* C = s_C + (zr & 1) * (3 * SNK * EY2);
         float* dst = s_fr + (size_t)(zr & (PSL - 1)) * (P2 * FENT);
         for (int k = tid; k < P2; k += NT) {
@@ -564,8 +578,58 @@ __device__ __forceinline__ void push_body(const PushArgs& pa, float* smem, int b
                 for (int c = 0; c < 3; ++c) acc[c] = __ffma2_rn(C[(c * SNK + kxi) * EY2 + ey], e, acc[c]);
             }
             const float Fx = acc[0].x + acc[0].y, Fy = acc[1].x + acc[1].y, Fz = acc[2].x + acc[2].y;
-            reinterpret_cast<float4*>(dst)[k] = make_float4(Fx, Fy, Fz, 0.f);
+            dst[3 * k] = Fx;
+            dst[3 * k + 1] = Fy;
+            dst[3 * k + 2] = Fz;
         }
+    };
+    // The band force along a column: F_c(z) = Re G_0 + Re(G_1 e^{iz}) + Re(G_2 e^{2iz}),
+    // G_kz = sum_kx D[c][kx][row][kz] e^{i kx x} of the column's (x, y): 15 real
+    // coefficients, made once per block for every column of the two-cell ring
+    auto fcolumns = [&]() {
+        for (int k = tid; k < P2; k += NT) {
+            const int ex = k % EX2, ey = k / EX2;
+            float G[3][5];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+#pragma unroll
+                for (int j = 0; j < 5; ++j) G[c][j] = 0.f;
+#pragma unroll
+                for (int kxi = 0; kxi < SNK; ++kxi) {
+                    const float2 e = s_tx2[kxi * EX2 + ex];
+                    const float2* D = s_D + ((c * SNK + kxi) * EY2 + ey) * 3;
+                    const float2 d0 = D[0], d1 = D[1], d2 = D[2];
+                    G[c][0] += d0.x * e.x + d0.y * e.y;
+                    G[c][1] += d1.x * e.x + d1.y * e.y;
+                    G[c][2] += d1.x * e.y - d1.y * e.x;
+                    G[c][3] += d2.x * e.x + d2.y * e.y;
+                    G[c][4] += d2.x * e.y - d2.y * e.x;
+                }
+            }
+            s_fc[k] = make_float4(G[0][0], G[1][0], G[2][0], G[0][1]);
+            s_fc[P2 + k] = make_float4(G[1][1], G[2][1], G[0][2], G[1][2]);
+            s_fc[2 * P2 + k] = make_float4(G[2][2], G[0][3], G[1][3], G[2][3]);
+            s_fc[3 * P2 + k] = make_float4(G[0][4], G[1][4], G[2][4], 0.f);
+        }
+    };
+    // band force of plane zr from them: a third of the table's instructions, for 20 KB more shared
+    // memory per block. That pays where no registers spill (single phase 256^3 603 -> 595 us per
+    // step, settle 713 -> 672, two-phase settle 128^3 111 -> 105); in the two-phase march the L1
+    // that it takes from the spill costs more (128^3 184 -> 204).
+    auto fsynth_columns = [&](int zr) {
+        float2 e1, e2;
+        ztw(zr, e1, e2);
+        float* dst = s_fr + (size_t)(zr & (PSL - 1)) * (P2 * FENT);
+        for (int k = tid; k < P2; k += NT) {
+            const float4 q0 = s_fc[k], q1 = s_fc[P2 + k], q2 = s_fc[2 * P2 + k], q3 = s_fc[3 * P2 + k];
+            dst[3 * k + 0] = fmaf(q0.w, e1.x, fmaf(q1.z, e1.y, fmaf(q2.y, e2.x, fmaf(q3.x, e2.y, q0.x))));
+            dst[3 * k + 1] = fmaf(q1.x, e1.x, fmaf(q1.w, e1.y, fmaf(q2.z, e2.x, fmaf(q3.y, e2.y, q0.y))));
+            dst[3 * k + 2] = fmaf(q1.y, e1.x, fmaf(q2.x, e1.y, fmaf(q2.w, e2.x, fmaf(q3.z, e2.y, q0.z))));
+        }
+    };
+    auto fsynth = [&](int zr) {
+        if constexpr (COLS) fsynth_columns(zr);
+        else fsynth_table(zr);
     };
     // c_i . F from a force-ring entry e (Fx, Fy, Fz), for direction i
     auto cFe = [](const float* e, int i) -> float {
@@ -574,8 +638,7 @@ __device__ __forceinline__ void push_body(const PushArgs& pa, float* smem, int b
             const float v = e[ax];
             return (cx(i) + cy(i) + cz(i)) > 0 ? v : -v;
         }
-        const float4 F = *reinterpret_cast<const float4*>(e);
-        return cdot3(i, F.x, F.y, F.z);
+        return cdot3(i, e[0], e[1], e[2]);
     };
 
     // ---- loads and moments ----
@@ -702,29 +765,32 @@ __device__ __forceinline__ void push_body(const PushArgs& pa, float* smem, int b
         if (fpend) {
             dtable();
             __syncthreads();
+            if (COLS) {
+                fcolumns();
+                __syncthreads();
+            }
         }
     }
     // band force planes of the prologue. Loading plane p reads F(p-1 .. p+1); the
-    // march (HALO) loads z0-1 and z0 here and the first iteration reads
-    // F(z0 .. z0+2) and synthesises F(z0+3) from C(z0+3); a settle loads z0 first.
-    // Four force slots and two table slots: a plane's table is written one barrier
-    // before its synthesis, a slot is rewritten only after its last reader's barrier.
+    // march loads z0-1 and z0 here and its first iteration reads F(z0 .. z0+2); a
+    // settle loads z0 first. Four force slots and two table slots: a plane's table
+    // is written one barrier before its synthesis, a slot is rewritten only after
+    // a barrier that follows its last reader.
     const int zlo = (HALO ? z0 - 1 : z0);  // first plane loaded
     if (fpend) {
         ctable(zlo - 1);
         ctable(zlo);
-        __syncthreads();
+        if (!COLS) __syncthreads();
         fsynth(zlo - 1);
         fsynth(zlo);
-        __syncthreads();
+        if (!COLS) __syncthreads();
         ctable(zlo + 1);
         ctable(zlo + 2);
-        __syncthreads();
+        if (!COLS) __syncthreads();
         fsynth(zlo + 1);
         if (HALO) fsynth(zlo + 2);
         __syncthreads();
-        // march (HALO): F(z0-2 .. z0+1) ready; F(z0+2), F(z0+3) follow the first loads.
-        // settle: F(z0-1 .. z0+1) ready, C(z0+2) waits in its slot.
+        // march: F(z0-2 .. z0+1) ready (without a ring F(z0-1 .. z0+1)); settle: F(z0-1 .. z0+1)
     }
     float bmin = INFINITY, bmax = -INFINITY;
     bool bad = false;
@@ -746,7 +812,12 @@ __device__ __forceinline__ void push_body(const PushArgs& pa, float* smem, int b
             bmin = fminf(bmin, ph);
             bmax = fmaxf(bmax, ph);
             bad |= !isfinite(dphi + dp + u1 + u2 + u3);
-            if (SPEC) {
+            if (UOUT) {
+                const unsigned s = (unsigned)zp * nxy + col;
+                a.maco[N + s] = u1;
+                a.maco[2 * N + s] = u2;
+                a.maco[3 * N + s] = u3;
+            } else if (SPEC) {
                 float2 e1, e2;
                 ztw(zp, e1, e2);
                 const float uu[3] = {u1, u2, u3};
@@ -836,12 +907,11 @@ __device__ __forceinline__ void push_body(const PushArgs& pa, float* smem, int b
     };
 
     if constexpr (SETTLE) {
-        // one plane at a time; before plane zp: F(zp+1) from C(zp+1), then C(zp+2)
+        // one plane at a time; before plane zp: F(zp+1)
         for (int zp = z0; zp < z1; ++zp) {
             if (fpend && zp > z0) {
                 __syncthreads();  // the previous plane's readers are done with the slot of F(zp-2)
                 fsynth(zp + 1);
-                ctable(zp + 2);
                 __syncthreads();
             }
             float v[2 * Q];
@@ -880,10 +950,10 @@ __device__ __forceinline__ void push_body(const PushArgs& pa, float* smem, int b
         own_plane(z0, A, oA[0], oA[1], oA[2], oA[3], oA[4]);
         halo_plane(z0);
         if (fpend) {
-            __syncthreads();  // the loads of z0-1 and z0 have read F(z0-2), F(z0-1) and C(z0), C(z0+1)
+            __syncthreads();  // the loads of z0-1 and z0 have read F(z0-2), F(z0-1) (and C(z0), C(z0+1))
             ctable(z0 + 2);
             ctable(z0 + 3);
-            __syncthreads();
+            if (!COLS) __syncthreads();
             fsynth(z0 + 2);
             fsynth(z0 + 3);
             __syncthreads();
@@ -928,7 +998,7 @@ __device__ __forceinline__ void push_body(const PushArgs& pa, float* smem, int b
         if (t < z1) iteration(t, A, B, oA, oB);
     }
 
-    if constexpr (SPEC) {
+    if constexpr (SPEC && !UOUT) {
         project_tile_sums(a, smem, s_tx1, s_ty1, cs, bx + 3 * by + 5 * bz);
         spectral_block_done(a, smem, nblk);
     }
@@ -951,6 +1021,15 @@ __global__ void __launch_bounds__(NT, 2) step_push(const __grid_constant__ PushA
     extern __shared__ __align__(128) float smem[];
     push_body<LES, FMODE, false, false, STG>(pa, smem, blockIdx.x, blockIdx.y, blockIdx.z,
                                              gridDim.x * gridDim.y * gridDim.z);
+}
+
+// band forcing with the projection as a launch of its own (project_chunks): the
+// step stores the u that it takes instead of summing it
+template <bool LES>
+__global__ void __launch_bounds__(NT, 2) step_push_u(const __grid_constant__ PushArgs pa) {
+    extern __shared__ __align__(128) float smem[];
+    push_body<LES, F_SPECTRAL, false, false, 0, true>(pa, smem, blockIdx.x, blockIdx.y, blockIdx.z,
+                                                      gridDim.x * gridDim.y * gridDim.z);
 }
 
 template <int FMODE, int STG>
@@ -1034,7 +1113,9 @@ static void push_args(dl_handle* h, PushArgs& pa, bool settle) {
     a.g = h->gs[c];
     a.fo = settle ? nullptr : h->fs[n];
     a.go = settle ? h->gs[c] : h->gs[n];
-    a.maco = settle ? h->mac32[c] : nullptr;
+    // (a push step leaves the fields stale: their buffer holds the stored u of step_push_u)
+    a.proj_in_step = settle || !chunked_projection(h);
+    a.maco = (settle || !a.proj_in_step) ? h->mac32[c] : nullptr;
     a.mac = nullptr;
     a.fh = h->fsp.d_fh[h->fsp.par];
     a.fh_next = h->fsp.d_fh[1 - h->fsp.par];
@@ -1109,8 +1190,19 @@ static int launch_push_t(dl_handle* h, const PushArgs& pa) {
     DL_CUDA(h, cudaGetLastError());
     return DL_OK;
 }
+template <bool LES>
+static int launch_push_u(dl_handle* h, const PushArgs& pa) {
+    static bool done[64] = {false};
+    const size_t sm = sizeof(float) * (size_t)push_smem_floats(true, false);
+    int rc = configure_smem(h, step_push_u<LES>, sm, done);
+    if (rc != DL_OK) return rc;
+    DL_LAUNCH(h, true, (step_push_u<LES><<<push_grid(h, pa.a.lz), NT, sm, h->stream>>>(pa)));
+    DL_CUDA(h, cudaGetLastError());
+    return launch_projection(h, pa.a);
+}
 template <bool LES, int FMODE>
 static int launch_push(dl_handle* h, const PushArgs& pa) {
+    if (FMODE == F_SPECTRAL && !pa.a.proj_in_step) return launch_push_u<LES>(h, pa);
     return h->push_bulk == 2   ? launch_push_t<LES, FMODE, 2>(h, pa)
            : h->push_bulk == 1 ? launch_push_t<LES, FMODE, 1>(h, pa)
                                : launch_push_t<LES, FMODE, 0>(h, pa);
@@ -1136,7 +1228,7 @@ static int launch_push_sp(dl_handle* h, const PushArgs& pa) {
 template <int FMODE, bool SP>
 static int launch_settle(dl_handle* h, const PushArgs& pa) {
     static bool done[64] = {false};
-    const size_t sm = sizeof(float) * (size_t)push_smem_floats(FMODE == F_SPECTRAL, SP);
+    const size_t sm = sizeof(float) * (size_t)push_smem_floats(FMODE == F_SPECTRAL, SP, 0, true);
     int rc = configure_smem(h, settle_push<FMODE, SP>, sm, done);
     if (rc != DL_OK) return rc;
     DL_LAUNCH(h, false, (settle_push<FMODE, SP><<<push_grid(h, pa.a.lz), NT, sm, h->stream>>>(pa)));
