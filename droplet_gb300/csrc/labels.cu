@@ -50,15 +50,18 @@ __device__ __forceinline__ bool fg(const LabelArgs& a, int s) {
 
 constexpr int LBL_MAXIT = 1 << 24;
 
-// the root of x; a walked site is moved up to its grandparent (a plain store: any
-// value written is an ancestor, so a racing reader only takes a longer way)
+// the root of x; HALVE: a walked site is moved up to its grandparent (a plain
+// store: any value written is an ancestor, so a racing reader only takes a longer
+// way). Not where sites get their final roots: a late store would put a site
+// that has its root back under an ancestor
+template <bool HALVE>
 __device__ __forceinline__ int find_root(const LabelArgs& a, int x) {
     int p = __ldcg(a.parent + x);
     for (int it = 0; it < LBL_MAXIT; ++it) {
         if (p == x) return x;
         const int g = __ldcg(a.parent + p);
         if (g == p) return p;
-        __stcg(a.parent + x, g);
+        if (HALVE) __stcg(a.parent + x, g);
         x = p;
         p = g;
     }
@@ -105,8 +108,8 @@ __global__ void __launch_bounds__(256) lbl_union(LabelArgs a) {
         }
         int u = s, v = t;
         for (int it = 0; it < LBL_MAXIT; ++it) {
-            u = find_root(a, u);
-            v = find_root(a, v);
+            u = find_root<true>(a, u);
+            v = find_root<true>(a, v);
             if (u == v) break;
             if (u < v) {
                 const int w = u;
@@ -126,7 +129,7 @@ __global__ void __launch_bounds__(256) lbl_compress_count(LabelArgs a) {
     const bool in = s < a.N && a.parent[s] >= 0;
     const unsigned who = __ballot_sync(0xffffffffu, in);
     if (!in) return;
-    const int r = find_root(a, s);
+    const int r = find_root<false>(a, s);
     a.parent[s] = r;
     const unsigned same = __match_any_sync(who, r);
     if ((threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(a.count + r, __popc(same));
