@@ -207,6 +207,7 @@ int fast_step(dl_handle* h);
 // push form (step_push.cu)
 bool push_tma_eligible(const dl_handle* h);
 bool push_eligible(const dl_handle* h);
+bool push_ranged(const dl_handle* h);
 int push_step(dl_handle* h);
 int fast_settle(dl_handle* h);  // complete a push step's state (no-op when settled)
 // the persistent ensemble launch in the push form (step_push.cu)
