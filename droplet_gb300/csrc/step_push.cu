@@ -747,7 +747,25 @@ __device__ __forceinline__ void push_body(const PushArgs& pa, float* smem, int b
         for (int i = 0; i < Q; ++i) v[Q + i] = s_pg[i * NT + tid];
     };
 
+    // the halo site's populations of plane zp into shared memory (asynchronous
+    // copies: no registers held while they arrive; each thread reads back its own)
+    auto issue_halo = [&](int zp) {
+        if (!has_h) return;
+        const unsigned s = (unsigned)wrap_near(zp, nz) * nxy + hcol;
+#pragma unroll
+        for (int i = 0; i < Q; ++i) cp_async4(s_h + i * NHALO + tid, (const float*)a.f + (unsigned)i * N + s);
+        if (NEEDG_HALO) {
+#pragma unroll
+            for (int i = 0; i < Q; ++i)
+                cp_async4(s_h + (Q + i) * NHALO + tid, (const float*)a.g + (unsigned)i * N + s);
+        }
+        cp_async_commit();
+    };
     // ---- prologue: band force tables and planes ----
+    // a staged march has its first plane arrive behind the tables (single phase 256^3
+    // 578 -> 570 us per step; into registers the same early loads gained nothing at
+    // any size and cost 96^3 1.3 %)
+    if (!SETTLE && BULK && !TMA) bulk_issue(z0 - 1);
     if (SPEC) {
         if (fpend) {
             for (int t = tid; t < SNK * EX2; t += NT) {
@@ -844,20 +862,6 @@ __device__ __forceinline__ void push_body(const PushArgs& pa, float* smem, int b
             }
         }
     };
-    // the halo site's populations of plane zp into shared memory (asynchronous
-    // copies: no registers held while they arrive; each thread reads back its own)
-    auto issue_halo = [&](int zp) {
-        if (!has_h) return;
-        const unsigned s = (unsigned)wrap_near(zp, nz) * nxy + hcol;
-#pragma unroll
-        for (int i = 0; i < Q; ++i) cp_async4(s_h + i * NHALO + tid, (const float*)a.f + (unsigned)i * N + s);
-        if (NEEDG_HALO) {
-#pragma unroll
-            for (int i = 0; i < Q; ++i)
-                cp_async4(s_h + (Q + i) * NHALO + tid, (const float*)a.g + (unsigned)i * N + s);
-        }
-        cp_async_commit();
-    };
     // the halo site's moments of plane zp into the ring, streamed pair by pair
     // from shared memory (band force of the sources, wall reflection, sums)
     auto halo_plane = [&](int zp) {
@@ -929,7 +933,7 @@ __device__ __forceinline__ void push_body(const PushArgs& pa, float* smem, int b
         }
         // planes zlo (= z0 - 1, moments only) and z0
         if (BULK) {
-            bulk_issue(z0 - 1);
+            if (TMA) bulk_issue(z0 - 1);
             issue_halo(z0 - 1);
             bulk_take(A);
         } else {
