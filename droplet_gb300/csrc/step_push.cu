@@ -70,10 +70,12 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // a population of the loaded state: read once per step, so it takes no L1 line
-// (L1 stays for the kernel's register spill, which it would otherwise evict)
-__device__ __forceinline__ float ld_stream(const float* p) {
+// (L1 stays for the kernel's register spill, which it would otherwise evict).
+// after: what after_previous_step returned; an operand the load does not use keeps
+// the compiler from moving it up past that wait without ordering it otherwise.
+__device__ __forceinline__ float ld_stream(const float* p, int after) {
     float v;
-    asm("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    asm("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p), "r"(after));
     return v;
 }
 
@@ -465,7 +467,8 @@ __device__ __forceinline__ void push_minmax(const FastArgs& a, float bmin, float
 // asynchronous copies, STG 1), or by one thread for the block (two tensor
 // copies completing on an mbarrier, STG 2; full tiles only)
 template <bool LES, int FMODE, bool SP, bool SETTLE, int STG = 0, bool UOUT = false>
-__device__ __forceinline__ void push_body(const PushArgs& pa, float* smem, int bx, int by, int bz, unsigned nblk) {
+__device__ __forceinline__ void push_body(const PushArgs& pa, float* smem, int bx, int by, int bz, unsigned nblk,
+                                          int after = 0) {
     constexpr bool BULK = STG != 0;
     constexpr bool TMA = STG == 2;
     constexpr bool SPEC = FMODE == F_SPECTRAL;
@@ -538,7 +541,7 @@ __device__ __forceinline__ void push_body(const PushArgs& pa, float* smem, int b
                 const int4 md = __ldg(a.modes + m);
                 if (md.z != kz) continue;
                 const float2 ey = s_ty2[(md.y + SK) * EY2 + yy];
-                const float2 fv = __ldg(a.fh + c * a.nm + m);
+                const float2 fv = a.fh[c * a.nm + m];
                 re += fv.x * ey.x - fv.y * ey.y;
                 im += fv.x * ey.y + fv.y * ey.x;
             }
@@ -647,11 +650,11 @@ __device__ __forceinline__ void push_body(const PushArgs& pa, float* smem, int b
         const unsigned s = (unsigned)wrap_near(zp, nz) * nxy + c;
         if (withf) {
 #pragma unroll
-            for (int i = 0; i < Q; ++i) v[i] = ld_stream((const float*)a.f + (unsigned)i * N + s);
+            for (int i = 0; i < Q; ++i) v[i] = ld_stream((const float*)a.f + (unsigned)i * N + s, after);
         }
         if (withg) {
 #pragma unroll
-            for (int i = 0; i < Q; ++i) v[Q + i] = ld_stream((const float*)a.g + (unsigned)i * N + s);
+            for (int i = 0; i < Q; ++i) v[Q + i] = ld_stream((const float*)a.g + (unsigned)i * N + s, after);
         }
     };
     // the pending part of the loaded g of the site at ring position (ex, ey) of plane zp:
@@ -1030,17 +1033,19 @@ __device__ __forceinline__ void push_body(const PushArgs& pa, float* smem, int b
 // an empty GPU, which a long march pays for: 96^3, lz 12, 53.9 -> 55.0, 128^3 LES and
 // band forcing, lz 32, 176 -> 180.
 constexpr int OVERLAP_LZ = 8;
-__device__ __forceinline__ void after_previous_step() {
-    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+__device__ __forceinline__ int after_previous_step() {
+    int after;
+    asm volatile("griddepcontrol.wait;\n\tmov.b32 %0, 0;\n" : "=r"(after)::"memory");
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    return after;
 }
 
 template <bool LES, int FMODE, int STG>
 __global__ void __launch_bounds__(NT, 2) step_push(const __grid_constant__ PushArgs pa) {
     extern __shared__ __align__(128) float smem[];
-    after_previous_step();
+    const int after = after_previous_step();
     push_body<LES, FMODE, false, false, STG>(pa, smem, blockIdx.x, blockIdx.y, blockIdx.z,
-                                             gridDim.x * gridDim.y * gridDim.z);
+                                             gridDim.x * gridDim.y * gridDim.z, after);
 }
 
 // band forcing with the projection as a launch of its own (project_chunks): the
@@ -1055,9 +1060,9 @@ __global__ void __launch_bounds__(NT, 2) step_push_u(const __grid_constant__ Pus
 template <int FMODE, int STG>
 __global__ void __launch_bounds__(NT, 2) step_push_sp(const __grid_constant__ PushArgs pa) {
     extern __shared__ __align__(128) float smem[];
-    after_previous_step();
+    const int after = after_previous_step();
     push_body<false, FMODE, true, false, STG>(pa, smem, blockIdx.x, blockIdx.y, blockIdx.z,
-                                              gridDim.x * gridDim.y * gridDim.z);
+                                              gridDim.x * gridDim.y * gridDim.z, after);
 }
 
 // an ensemble's push steps as ONE persistent launch: work items (member, tile
