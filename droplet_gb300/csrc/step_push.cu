@@ -71,11 +71,16 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 
 // a population of the loaded state: read once per step, so it takes no L1 line
 // (L1 stays for the kernel's register spill, which it would otherwise evict).
+// A coherent load, not the .nc of read-only data: the blocks of an overlapped step
+// (after_previous_step) are resident while the step before it still writes these
+// arrays, and a settle stores g where it loaded it. The same holds for everything
+// else that a step's predecessor writes (coefficients, range); __ldg is for what no
+// step writes (modes, twiddles, a static force).
 // after: what after_previous_step returned; an operand the load does not use keeps
 // the compiler from moving it up past that wait without ordering it otherwise.
 __device__ __forceinline__ float ld_stream(const float* p, int after) {
     float v;
-    asm("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p), "r"(after));
+    asm("ld.global.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p), "r"(after));
     return v;
 }
 
