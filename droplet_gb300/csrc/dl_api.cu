@@ -670,6 +670,7 @@ int dl_set_populations(dl_handle* h, const double* f, const double* g) {
         DL_CUDA(h, cudaMemcpyAsync(st.d + Q * h->N, g, bytes, cudaMemcpyHostToDevice, h->stream));
         int rc = fast_set_populations(h, st.d, st.d + Q * h->N);
         if (rc != DL_OK) return rc;
+        h->pushed = 0;  // complete, whatever the replaced state awaited
         DL_CUDA(h, cudaStreamSynchronize(h->stream));
         h->fields_set = true;
         h->eq_init = true;
