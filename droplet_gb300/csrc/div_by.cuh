@@ -82,21 +82,33 @@ static __host__ __device__ __noinline__ double div_general(double x, double y) {
 inline double div_general(double x, double y) { return x / y; }
 #endif
 
+// q with the sign of x, which every quotient by a positive divisor has: of x = -0 the
+// additions make +0 (zl < 0, or a remainder of +0)
+DL_HD double div_signed(double q, double x) {
+#if defined(__CUDA_ARCH__)
+    return __hiloint2double(__double2hiint(q) | (__double2hiint(x) & (int)0x80000000u), __double2loint(q));
+#else
+    return copysign(q, x);
+#endif
+}
+
+DL_HD double div_short(double x, double zh, double zl) { return div_signed(div_fma(x, zh, x * zl), x); }
+
 DL_HD double div_correct(double x, double y, double zh, double zl) {
     const double q = div_fma(x, zh, x * zl);
-    return div_fma(div_fma(-q, y, x), zh, q);
+    return div_signed(div_fma(div_fma(-q, y, x), zh, q), x);
 }
 
 DL_HD double div_markstein(double x, double y, double zh) {
     const double q = x * zh;
-    return div_fma(div_fma(-q, y, x), zh, q);
+    return div_signed(div_fma(div_fma(-q, y, x), zh, q), x);
 }
 
 DL_HD double div_by(double x, const DivBy& d) {
     if (d.how == DIV_ONE) return x;
     if (d.how == DIV_GENERAL || !div_numerator_ok(x)) return div_general(x, d.y);
     if (d.how == DIV_CORRECT) return div_correct(x, d.y, d.zh, d.zl);
-    if (d.how == DIV_SHORT) return div_fma(x, d.zh, x * d.zl);
+    if (d.how == DIV_SHORT) return div_short(x, d.zh, d.zl);
     if (d.how == DIV_EXACT) return x * d.zh;
     return div_markstein(x, d.y, d.zh);
 }
