@@ -1530,6 +1530,25 @@ static int batch_lz(BatchImpl* b) {
     return b->lz_auto[c] = best;
 }
 
+// the members' "lz" during a batched step: the batch's. A member's own setting is
+// put back after it, for its steps outside the batch
+struct BatchPlanes {
+    BatchImpl* b;
+    std::vector<int> own;
+    explicit BatchPlanes(BatchImpl* batch) : b(batch), own(batch->nm) {
+        const int lz = batch_lz(b);
+        for (int m = 0; m < b->nm; ++m) {
+            own[m] = b->mem[m]->lz;
+            b->mem[m]->lz = std::min(lz, b->mem[m]->nz);
+        }
+    }
+    ~BatchPlanes() {
+        for (int m = 0; m < b->nm; ++m) b->mem[m]->lz = own[m];
+    }
+    BatchPlanes(const BatchPlanes&) = delete;
+    BatchPlanes& operator=(const BatchPlanes&) = delete;
+};
+
 template <typename ST, bool RES, bool LES, int FMODE>
 static int launch_batched_t(dl_handle* h0, BatchImpl* b, int k) {
     static bool configured[64] = {false};
@@ -1630,7 +1649,7 @@ void batch_destroy(void* p) {
 int batch_set_option(void* p, const char* key, long long v) {
     BatchImpl* b = (BatchImpl*)p;
     if (strcmp(key, "lz") == 0) {
-        if (v < 1 || v > 4096) return DL_ERR_ARG;
+        if (v < 0 || v > 4096) return DL_ERR_ARG;  // 0: chosen by batch_lz
         b->lz = (int)v;
     } else if (strcmp(key, "blocks_per_sm") == 0) {
         if (v < 1 || v > 2) return DL_ERR_ARG;
@@ -1678,8 +1697,7 @@ static int batch_build(BatchImpl* b) {
         DL_CUDA(h0, cudaMalloc(&b->d_counter, sizeof(unsigned)));
     }
     for (int m = 0; m < nm; ++m) {
-        dl_handle* h = b->mem[m];
-        h->lz = min(batch_lz(b), h->nz);
+        dl_handle* h = b->mem[m];  // (h->lz: BatchPlanes)
         for (int k = 0; k < 2; ++k) {
             if (b->push) {
                 push_args_at(h, k, b->h_ptable + ((size_t)k * nm + m) * psz);  // the projection is in the push body
@@ -1791,11 +1809,10 @@ static int batch_step_concurrent(BatchImpl* b, int nsteps) {
             DL_CUDA(h0, cudaStreamWaitEvent(b->workers[m % nw], b->fork, 0));
         }
     int rc = DL_OK;
-    const int lz = batch_lz(b);
+    const BatchPlanes planes(b);
     for (int s = 0; s < nsteps && rc == DL_OK; ++s)
         for (int m = 0; m < nm && rc == DL_OK; ++m) {
             dl_handle* h = b->mem[m];
-            h->lz = std::min(lz, h->nz);
             cudaStream_t own = h->stream;
             h->stream = b->workers[m % nw];
             rc = fast_step(h);
@@ -1827,6 +1844,7 @@ int batch_step(void* p, int nsteps) {
         if (h->P.walls && h->P.wall_start > h->step + 1 && h->P.wall_start <= h->step + nsteps)
             return set_error(h0, DL_ERR_UNSUPPORTED, "wall start inside a batched call; split the call");
     }
+    const BatchPlanes planes(b);
     // the push form when every member takes it (FP32 members); else the pull form
     bool push = true;
     for (int m = 0; m < nm; ++m) push = push && push_eligible(b->mem[m]);

@@ -399,10 +399,10 @@ int dl_batch_set_stream(dl_batch* b, void* cuda_stream);
 int dl_batch_step(dl_batch* b, int nsteps);
 
 /* Knobs: "persistent" 0|1 (the mode above, default 0); "lz" z planes per
- * block or work item (at most a member's nz; until it is set, chosen from the
- * members' sizes); "blocks_per_sm"
- * persistent blocks per SM (1 or 2); "graph" 1 = replay step pairs of the
- * persistent launch from a CUDA graph. */
+ * block or work item (at most a member's nz; 0, the default: chosen from the
+ * members' sizes; a member's own "lz" holds for its steps outside the batch);
+ * "blocks_per_sm" persistent blocks per SM (1 or 2); "graph" 1 = replay step
+ * pairs of the persistent launch from a CUDA graph. */
 int dl_batch_set_option(dl_batch* b, const char* key, int64_t value);
 int dl_batch_get_option(dl_batch* b, const char* key, int64_t* value);
 
