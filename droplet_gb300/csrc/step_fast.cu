@@ -1478,8 +1478,8 @@ struct BatchImpl {
     int2* d_pitems;         // projection work items (member, row block)
     unsigned* d_pnblk;      // projection blocks per member
     int npitems;
-    int lz, bps, use_graph; // lz 0: chosen by batch_lz
-    int lz_auto[3];         // that choice by prologue class (0: not made yet)
+    int lz, bps, use_graph; // lz 0: chosen by member_lz
+    int lz_auto;            // batch_lz's choice (0: not made yet)
     int persistent;         // 1: one persistent launch per step over all members; 0: the members' own steps, concurrent
     int nworkers;           // concurrent mode: worker streams (created on first use)
     cudaStream_t workers[BATCH_WORKERS];
@@ -1498,22 +1498,21 @@ struct BatchImpl {
     unsigned* d_counter;    // push form: the launch's next work item
 };
 
-// One lz for all members. Their launches overlap, so there are no common waves:
-// the cost is every block's planes and prologue (4.5 planes here) over the
-// 2 x SMs slots, and a quarter of a block for the end of the step, where few
-// are left; at least one block's time. Measured (us per step at the constant 32
-// before / at the choice): 64 members of 48^3 .. 96^3 1884 / 1845, 16 members
-// 624 / 612, two of 96^3 183 / 149. FP16 members with band forcing keep
-// BAND_CHUNK (its sums are grouped by chunk, see project_chunks).
+// One lz for all members without a two-phase band force. Their launches overlap,
+// so there are no common waves: the cost is every block's planes and prologue (4.5
+// planes here) over the 2 x SMs slots, and a quarter of a block for the end of the
+// step, where few are left; at least one block's time. Measured with moving walls (us
+// per step at a constant 32 / at the choice): FP32 four members of 40^3 69 / 28 (lz
+// 6), four of 64^3 92 / 64, two of 96^3 118 / 107, 64 of 48^3 .. 96^3 1836 / 1856
+// (lz 48, where shorter marches are better by up to 4 %); FP16 the last 1860 / 1844.
 static int batch_lz(BatchImpl* b) {
     if (b->lz > 0) return b->lz;
-    const int c = prologue_class(b->mem[0]);
-    if (b->lz_auto[c]) return b->lz_auto[c];
+    if (b->lz_auto) return b->lz_auto;
     int nzmax = 1;
     for (int m = 0; m < b->nm; ++m) nzmax = std::max(nzmax, b->mem[m]->nz);
     int best = BAND_CHUNK;
     double cost = INFINITY;
-    for (int k = (nzmax + 63) / 64; k <= nzmax && !band_two_phase(b->mem[0]); ++k) {  // at most 64 planes
+    for (int k = (nzmax + 63) / 64; k <= nzmax; ++k) {  // at most 64 planes
         const int lz = (nzmax + k - 1) / k;
         double planes = 0.0;
         for (int m = 0; m < b->nm; ++m) {
@@ -1527,7 +1526,15 @@ static int batch_lz(BatchImpl* b) {
             best = lz;
         }
     }
-    return b->lz_auto[c] = best;
+    return b->lz_auto = best;
+}
+
+// the planes per block of member h: a two-phase member with band forcing keeps
+// BAND_CHUNK unless the batch's "lz" is set, because its FP32 band sums are grouped
+// by block (see project_chunks), whatever the other members do
+static int member_lz(BatchImpl* b, const dl_handle* h) {
+    const int lz = b->lz > 0 ? b->lz : band_two_phase(h) ? BAND_CHUNK : batch_lz(b);
+    return std::min(lz, h->nz);
 }
 
 // the members' "lz" during a batched step: the batch's. A member's own setting is
@@ -1536,10 +1543,9 @@ struct BatchPlanes {
     BatchImpl* b;
     std::vector<int> own;
     explicit BatchPlanes(BatchImpl* batch) : b(batch), own(batch->nm) {
-        const int lz = batch_lz(b);
         for (int m = 0; m < b->nm; ++m) {
             own[m] = b->mem[m]->lz;
-            b->mem[m]->lz = std::min(lz, b->mem[m]->nz);
+            b->mem[m]->lz = member_lz(b, b->mem[m]);
         }
     }
     ~BatchPlanes() {
@@ -1649,7 +1655,7 @@ void batch_destroy(void* p) {
 int batch_set_option(void* p, const char* key, long long v) {
     BatchImpl* b = (BatchImpl*)p;
     if (strcmp(key, "lz") == 0) {
-        if (v < 0 || v > 4096) return DL_ERR_ARG;  // 0: chosen by batch_lz
+        if (v < 0 || v > 4096) return DL_ERR_ARG;  // 0: chosen by member_lz
         b->lz = (int)v;
     } else if (strcmp(key, "blocks_per_sm") == 0) {
         if (v < 1 || v > 2) return DL_ERR_ARG;
@@ -1668,7 +1674,7 @@ int batch_set_option(void* p, const char* key, long long v) {
 
 int batch_get_option(void* p, const char* key, long long* v) {
     BatchImpl* b = (BatchImpl*)p;
-    if (strcmp(key, "lz") == 0) *v = batch_lz(b);
+    if (strcmp(key, "lz") == 0) *v = (b->lz == 0 && band_two_phase(b->mem[0])) ? BAND_CHUNK : batch_lz(b);
     else if (strcmp(key, "blocks_per_sm") == 0) *v = b->bps;
     else if (strcmp(key, "graph") == 0) *v = b->use_graph;
     else if (strcmp(key, "persistent") == 0) *v = b->persistent;
