@@ -593,37 +593,24 @@ __global__ void mirror_copy(const DevState* __restrict__ st, double* __restrict_
     }
 }
 
-// A viscosity ratio with the previous step's phi range takes the push form
-// (push_ranged) in calls of at least RANGED_STEPS on at least RANGED_SITES: such a
-// call ends with a settle, half a step, and each step has phi_range's launch,
-// some 8 us where the domain is small. us per call, pull / push: 150 x 101 x 77 4
-// steps 552 / 450, 20 steps 2748 / 2063; 64^3 4 steps 124 / 120; 24^3 4 steps 50 /
-// 66. Every call with a host mirror of the range, which the pull form has right
-// after each step, stays there.
-constexpr int RANGED_STEPS = 4;
-constexpr size_t RANGED_SITES = 1 << 18;
-
 int dl_step(dl_handle* h, int nsteps) {
     if (!h || nsteps < 0) return DL_ERR_ARG;
     if (!h->eq_init) return set_error(h, DL_ERR_STATE, "dl_step before dl_init_equilibrium / dl_set_populations");
-    if (is_fast(h) && nsteps >= RANGED_STEPS && h->N >= RANGED_SITES && !h->mirror_dev && push_ranged(h)) {
-        for (int k = 0; k < nsteps; ++k) {
-            const int rc = push_step(h);
-            if (rc != DL_OK) return rc;
-        }
-        return fast_settle(h);
-    }
+    const bool ranged = is_fast(h) && push_ranged(h);
     for (int k = 0; k < nsteps; ++k) {
         int rc = is_fast(h) ? fast_step(h) : fp64_step(h);
         if (rc != DL_OK) return rc;
         if (h->mirror_dev) {
-            // a push step reduces the range of the state it loaded, the previous step's
-            const long long at = h->pushed ? h->step - 1 : h->step;
+            // a push step reduces the range of the state it loaded, the previous step's; a
+            // ranged one's own is taken here, for the next step too, or by the last settle
+            if (ranged) rc = k < nsteps - 1 ? push_range(h) : fast_settle(h);
+            if (rc != DL_OK) return rc;
+            const long long at = h->pushed && !ranged ? h->step - 1 : h->step;
             DL_LAUNCH(h, false, (mirror_copy<<<1, 32, 0, h->stream>>>(h->d_state, h->mirror_dev, at & h->mirror_mask)));
             DL_CUDA(h, cudaGetLastError());
         }
     }
-    return DL_OK;
+    return ranged ? fast_settle(h) : DL_OK;
 }
 
 int dl_get_populations(dl_handle* h, double* f, double* g) {

@@ -142,6 +142,7 @@ struct dl_handle {
     int proj_in_step;        // band forcing: projection of the new u inside the fused step (else its own launch)
     int push;                // FP32: step in the push form where eligible (option "push")
     int pushed;              // the state is a push step's: fields stale, band force and wall reflection pending
+    int range_known;         // pushed: the device state has the phi range of this state (push_range)
     int push_bulk;           // push form: next plane staged in shared memory (option "stage": 0 registers,
                              // 1 per-thread asynchronous copies, 2 tensor copies, full tiles only)
     unsigned char push_tmap[4][128];  // stage 2: tensor maps of fs[0], fs[1], gs[0], gs[1]
@@ -208,6 +209,7 @@ int fast_step(dl_handle* h);
 bool push_tma_eligible(const dl_handle* h);
 bool push_eligible(const dl_handle* h);
 bool push_ranged(const dl_handle* h);
+int push_range(dl_handle* h);  // the phi range of a ranged push step's state
 int push_step(dl_handle* h);
 int fast_settle(dl_handle* h);  // complete a push step's state (no-op when settled)
 // the persistent ensemble launch in the push form (step_push.cu)

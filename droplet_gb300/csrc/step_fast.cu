@@ -1018,7 +1018,7 @@ static bool band_two_phase(const dl_handle* h) {
     return force_fmode(h) == F_SPECTRAL && (!h->single || h->form == DL_FORM_FP16);
 }
 // step_push_u has no staged variants
-static bool has_chunked_step(const dl_handle* h) { return !(push_eligible(h) && h->push_bulk != 0); }
+static bool has_chunked_step(const dl_handle* h) { return !((push_eligible(h) || push_ranged(h)) && h->push_bulk != 0); }
 
 int effective_lz(dl_handle* h) {
     if (h->lz > 0) return h->lz;
@@ -1394,7 +1394,7 @@ void advance(dl_handle* h, int n) {
 }
 
 int fast_step(dl_handle* h) {
-    if (push_eligible(h)) return push_step(h);
+    if (push_eligible(h) || push_ranged(h)) return push_step(h);
     if (h->pushed) {
         const int src = fast_settle(h);
         if (src != DL_OK) return src;
@@ -1822,6 +1822,7 @@ static int batch_step_concurrent(BatchImpl* b, int nsteps) {
             cudaStream_t own = h->stream;
             h->stream = b->workers[m % nw];
             rc = fast_step(h);
+            if (rc == DL_OK && s == nsteps - 1 && push_ranged(h)) rc = fast_settle(h);  // as dl_step leaves it
             h->stream = own;
         }
     // join even after an error, so that the home stream (and a member's own stream)

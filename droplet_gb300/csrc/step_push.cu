@@ -41,9 +41,9 @@
 // copies per plane (TMA, box 32 x 8 x 1 x 15 of the f and g arrays) that
 // complete on an mbarrier (2).
 //
-// Eligible: FP32 storage, viscosity ratio 1 or the fixed-viscosity mode (the
-// step's tau_g then needs no phi range of the state it collides), band
-// forcing with kc <= 3 or no band forcing.
+// Eligible: FP32 storage, band forcing with kc <= 3 or no band forcing, and a tau_g
+// that needs no phi range of the state that the step collides (viscosity ratio 1 or
+// the fixed-viscosity mode), or whose range a pass before the step takes (push_ranged).
 #include "fast_common.cuh"
 
 #include <cuda.h>  // CUtensorMap and the encoder's enums (the encoder is resolved at run time)
@@ -534,7 +534,7 @@ __device__ __forceinline__ void push_body(const PushArgs& pa, float* smem, int b
         mn = (float)a.st->phi_min;
         mx = (float)a.st->phi_max;
     }
-    const float kscale = a.dnu / (mx - mn);  // zero: eligible only with nu2 = nu1 or the fixed mode
+    const float kscale = a.dnu / (mx - mn);  // (range of the loaded state: push_ranged)
 
     // ---- band force tables (pending band force) ----
     auto dtable = [&]() {
@@ -1148,12 +1148,20 @@ __global__ void __launch_bounds__(RANGE_NT) phi_range(const FastArgs a) {
 }
 
 // ---- host side ------------------------------------------------------------------
-// steps of one call can take the push form although tau_g needs the phi range of
-// the state being collided: phi_range before each, a settle after the last
+// A viscosity ratio with the range of the previous step's phi: the push form with
+// phi_range before each step of a pending state, on RANGED_SITES or more (phi_range's
+// launch takes some 8 us where the domain is small). Which form a step takes depends
+// on the handle alone, not on how many steps a call has, what reads the state between
+// them or which ensemble the handle is in: the forms round differently.
+// A call ends settled. us per step in calls of 1 / 4 / 20 steps, pull form: 150 x 101
+// x 77 120 / 120 / 120, 128^3 186 / 186 / 187; this one: 142 / 109 / 100, 203 / 166 /
+// 156. A host that steps one by one and keeps the state settled is better off in the
+// pull form (option "push" 0).
+constexpr size_t RANGED_SITES = 1 << 18;
 bool push_ranged(const dl_handle* h) {
     const dl_params& P = h->P;
     return h->form == DL_FORM_FP32 && h->push && !h->single && P.nu2 != P.nu1 && P.visc_mode != DL_VISC_FIXED &&
-           !(h->force_mode == DL_FORCE_SPECTRAL && h->fsp.nm == 0);
+           !(h->force_mode == DL_FORCE_SPECTRAL && h->fsp.nm == 0) && h->N >= RANGED_SITES;
 }
 
 bool push_eligible(const dl_handle* h) {
@@ -1318,16 +1326,25 @@ static int launch_settle(dl_handle* h, const PushArgs& pa) {
     return DL_OK;
 }
 
-int push_step(dl_handle* h) {
+int push_range(dl_handle* h) {
+    if (!h->pushed || h->range_known) return DL_OK;  // a settled state's is in the device state
     PushArgs pa;
     push_args(h, pa, false);
-    if (h->pushed && push_ranged(h)) {  // a settled state's range is in the device state
-        FastArgs r = pa.a;
-        r.maco = h->mac32[h->cur];  // stale in a pushed state
-        const unsigned grid = (unsigned)std::min<size_t>((h->N + RANGE_NT - 1) / RANGE_NT, 8 * (size_t)sm_count(h));
-        DL_LAUNCH(h, false, (phi_range<<<grid, RANGE_NT, 0, h->stream>>>(r)));
-        DL_CUDA(h, cudaGetLastError());
+    pa.a.maco = h->mac32[h->cur];  // stale in a pushed state
+    const unsigned grid = (unsigned)std::min<size_t>((h->N + RANGE_NT - 1) / RANGE_NT, 8 * (size_t)sm_count(h));
+    DL_LAUNCH(h, false, (phi_range<<<grid, RANGE_NT, 0, h->stream>>>(pa.a)));
+    DL_CUDA(h, cudaGetLastError());
+    h->range_known = 1;
+    return DL_OK;
+}
+
+int push_step(dl_handle* h) {
+    if (push_ranged(h)) {
+        const int rc = push_range(h);
+        if (rc != DL_OK) return rc;
     }
+    PushArgs pa;
+    push_args(h, pa, false);
     if (h->push_bulk == 2) {
         const int rc = make_tmaps(h);
         if (rc != DL_OK) return rc;
@@ -1354,6 +1371,7 @@ int push_step(dl_handle* h) {
     if (rc != DL_OK) return rc;
     advance(h, 1);  // the launch wrote the next band coefficients (from the u it loaded)
     h->pushed = 1;
+    h->range_known = 0;
     h->fsp.dirty = 0;
     return DL_OK;
 }

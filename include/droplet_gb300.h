@@ -302,7 +302,12 @@ int dl_profile_read(dl_handle* h, dl_profile_stats* out);
  * each block of the fused step after its march, else by a launch of its own;
  * both give the same coefficients up to the FP32 summation order. "push" 0|1
  * (FP32, default 1): step in the push form where eligible (read-only keys
- * "push_eligible" and "pushed" report it). "stage" (push form) 0: the next
+ * "push_eligible" and "pushed" report it). A viscosity ratio with the range of
+ * the previous step's phi takes it too ("push_eligible" stays 0) on 2^18 sites
+ * or more, whatever the number of steps in a call; such a call ends settled
+ * ("pushed" 0), and the persistent batch launch steps such members in the pull
+ * form. The forms round differently; "push" = 0 gives the pull form everywhere.
+ * "stage" (push form) 0: the next
  * plane's populations loaded into registers (two-phase default); 1: staged in
  * shared memory by per-thread asynchronous copies (single-phase default); 2:
  * staged by two tensor (TMA) copies per plane completing on an mbarrier
