@@ -419,7 +419,8 @@ __device__ __forceinline__ void tile_twiddles(const FastArgs& a, float2* s_tx, f
 // (e^{i ky y}) are the block's halo-indexed twiddle tables.
 constexpr int PT_NV = 15;  // column values: per component sum u, Re/Im sum u e^{-iz}, Re/Im sum u e^{-2iz}
 constexpr int PT_NR = SNK * 3 * 3 * TY;  // row sums (kx, c, kz, row), complex
-constexpr int PT_SCRATCH = PT_NV * NT + 2 * PT_NR + 2 * FIN_SCRATCH;
+constexpr int PT_SUMS = PT_NV * NT + 2 * PT_NR;  // what is formed with the twiddle tables at hand
+constexpr int PT_SCRATCH = PT_SUMS + 2 * FIN_SCRATCH;
 static_assert(3 * 3 * 3 * TY <= NT, "one row sum of kx >= 0 per thread");
 
 // this thread's column sums over z of the new u it wrote (planes z0 .. z1-1):
@@ -542,7 +543,7 @@ __device__ __forceinline__ void spectral_block_done(const FastArgs& a, float* sc
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    spectral_finalize(a, reinterpret_cast<double*>(scr + PT_NV * NT + 2 * PT_NR));
+    spectral_finalize(a, reinterpret_cast<double*>(scr + PT_SUMS));
     if (threadIdx.x == 0) a.st->sp_done = 0u;
 }
 

@@ -161,7 +161,17 @@ __host__ __device__ constexpr int push_stage_offset(bool spec, bool sp) { return
 __host__ __device__ constexpr int push_smem_floats(bool spec, bool sp, int stage = 0, bool settle = false) {
     return stage == 0 ? push_rings_floats(spec, sp, sp || settle) : push_stage_offset(spec, sp) + pb_floats(sp) + (stage == 2 ? 36 : 0);
 }
-static_assert(PSL * P1 * 4 + PSL * P2 * FENT >= PT_SCRATCH, "projection scratch exceeds the rings");
+// The projection's scratch starts where the rings do. Its sums are formed with the
+// tables s_tx1, s_ty1, which follow the rings: they must end below them. What the last
+// block adds to turn them into coefficients comes after the tables' last use and may
+// lie over them (in a single-phase block it does: 5,184 floats of rings, 5,474 of
+// scratch), not past the block's memory.
+constexpr int push_tables_offset(bool sp) { return (sp ? 0 : PSL * P1 * 4 + 2 * Q * NHALO) + PSL * P2 * FENT; }
+static_assert(PT_SUMS <= push_tables_offset(false) && PT_SUMS <= push_tables_offset(true),
+              "projection sums over the tables that they are formed with");
+static_assert(PT_SCRATCH <= push_rings_floats(true, false, false) && PT_SCRATCH <= push_rings_floats(true, false, true) &&
+                  PT_SCRATCH <= push_rings_floats(true, true, true),
+              "projection scratch past the block's shared memory");
 
 // ring position (1-cell halo coordinates ex, ey in [0, EX1) x [0, EY1)) of the
 // thread's halo site h = 0 .. NHALO-1
@@ -484,7 +494,7 @@ __device__ __forceinline__ void push_body(const PushArgs& pa, float* smem, int b
     float4* s_mom = reinterpret_cast<float4*>(smem);              // [PSL][P1] (dphi, u1, u2, u3)
     float* s_h = smem + PSL * P1 * 4;                              // [2 Q][NHALO] halo sites' populations
     float* s_fr = smem + (SP ? 0 : PSL * P1 * 4 + 2 * Q * NHALO);  // [PSL][P2][FENT]
-    float2* s_tx1 = reinterpret_cast<float2*>(s_fr + PSL * P2 * FENT);  // [SNK][EX1] projection tables
+    float2* s_tx1 = reinterpret_cast<float2*>(smem + push_tables_offset(SP));  // [SNK][EX1] projection tables
     float2* s_ty1 = s_tx1 + SNK * EX1;                             // [SNK][EY1]
     float4* s_fc = reinterpret_cast<float4*>(s_ty1 + SNK * EY1);   // COLS: [FCOL][P2] columns' coefficients
     // the tables of the per-plane synthesis; with COLS they are only used while the
