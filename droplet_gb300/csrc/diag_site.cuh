@@ -29,28 +29,51 @@ struct DiagConsts {
     double phi1, phi_off, p_off;  // stored phi and p are phi - phi_off, p - p_off
     double inv_span, mid, nu1, dnu;
     double sfac;  // 1 / (4 graddiv^2)
-    int chunk;    // planes a block marches at a time (diag_chunk)
+    int ltx, chunk;  // diag_march
 };
 
-// blocks of DIAG_NT threads walk 32 x 8 column tiles
-constexpr int DIAG_TX = 32, DIAG_TY = 8, DIAG_NT = DIAG_TX * DIAG_TY;
-constexpr int DIAG_EX = DIAG_TX + 2, DIAG_P = DIAG_EX * (DIAG_TY + 2);
+// Blocks of DIAG_NT threads walk tiles of 2^ltx x (256 / 2^ltx) columns, some planes
+// at a time. The FP64 pipe is the bound of these marches and takes a warp's
+// instruction whole however few of its lanes have a site: the tile is 32 wide unless a
+// narrower one, whose warps take two, four or eight rows, has at least 5 % fewer
+// warps with a site (sides just above a multiple of 32, or below 32; with fewer
+// warps to save the chunks' split of the planes decides: 150 x 101 x 77 is 9 % slower
+// 8 wide, with 2 % fewer). us at 32 wide / at the choice, reduction of FP64 fields and
+// free energy of FP32 ones: 8 x 512 x 512 2117 / 549, 1299 / 346; 33 x 256 x 256 1147 /
+// 645, 681 / 393; 100 x 128 x 128 609 / 493, 348 / 299; 128^3 608, 348 at any width.
+constexpr int DIAG_NT = 256, DIAG_LMIN = 2;
+constexpr int DIAG_P = ((1 << DIAG_LMIN) + 2) * ((DIAG_NT >> DIAG_LMIN) + 2);  // ring positions of the narrowest tile, the most
+
+inline int diag_tile(int nx, int ny) {
+    auto warps = [&](int l) { return (long long)((nx + (1 << l) - 1) >> l) * ((ny + (32 >> l) - 1) / (32 >> l)); };
+    int best = 5;
+    for (int l = 4; l >= DIAG_LMIN; --l)
+        if (20 * warps(l) <= 19 * warps(best)) best = l;
+    return best;
+}
+inline long long diag_tiles(int nx, int ny, int ltx) {
+    const int ty = DIAG_NT >> ltx;
+    return (long long)((nx + (1 << ltx) - 1) >> ltx) * ((ny + ty - 1) / ty);
+}
 
 // planes per tile chunk for nblocks blocks: the even split of nz with the least
-// rounds x (planes + the ring planes' loads and the fold of the moments)
-inline int diag_chunk(int nx, int ny, int nz, int nblocks) {
-    const long long tiles = (long long)((nx + DIAG_TX - 1) / DIAG_TX) * ((ny + DIAG_TY - 1) / DIAG_TY);
+// rounds x (planes + extra, for the ring planes' loads and what follows a chunk)
+inline int diag_chunk(long long tiles, int nz, int nblocks, double extra) {
     int best = 1;
     double cost = 1e300;
     for (int m = 1; m <= nz; ++m) {
         const int c = (nz + m - 1) / m;
-        const double t = (double)((tiles * ((nz + c - 1) / c) + nblocks - 1) / nblocks) * (c + 1.0);
+        const double t = (double)((tiles * ((nz + c - 1) / c) + nblocks - 1) / nblocks) * (c + extra);
         if (t < cost) {
             cost = t;
             best = c;
         }
     }
     return best;
+}
+inline void diag_march(DiagConsts& k, int nblocks) {
+    k.ltx = diag_tile(k.nx, k.ny);
+    k.chunk = diag_chunk(diag_tiles(k.nx, k.ny, k.ltx), k.nz, nblocks, 1.0);
 }
 
 // the constants for handle h (reduce.cu)
@@ -86,10 +109,10 @@ __device__ __forceinline__ float diag_max(float a, float b) { return fmaxf(a, b)
 __device__ __forceinline__ double diag_min(double a, double b) { return fmin(a, b); }
 __device__ __forceinline__ double diag_max(double a, double b) { return fmax(a, b); }
 
-// site s of plane z, at ring position p of planes m, c, n (z - 1, z, z + 1)
+// site s of plane z, at ring position p (rows ex apart) of planes m, c, n (z - 1, z, z + 1)
 template <typename T>
 __device__ __forceinline__ void diag_site(const T (&m)[3][DIAG_P], const T (&c)[3][DIAG_P], const T (&n)[3][DIAG_P],
-                                          int p, T v, T dpT, const DiagConsts& k, int z, DiagAcc<T>& a) {
+                                          int p, int ex, T v, T dpT, const DiagConsts& k, int z, DiagAcc<T>& a) {
     const double u1 = (double)c[0][p], u2 = (double)c[1][p], u3 = (double)c[2][p];
     const double dp = (double)dpT;
     const double ph = k.phi_off + (double)v;
@@ -100,7 +123,7 @@ __device__ __forceinline__ void diag_site(const T (&m)[3][DIAG_P], const T (&c)[
 #pragma unroll
     for (int i = 1; i < Q; ++i) {
         const T(&r)[3][DIAG_P] = cz(i) < 0 ? m : (cz(i) > 0 ? n : c);
-        const int q = p + cy(i) * DIAG_EX + cx(i);
+        const int q = p + cy(i) * ex + cx(i);
         const T w[3] = {r[0][q], r[1][q], r[2][q]};
         const int cc[3] = {cx(i), cy(i), cz(i)};
 #pragma unroll
@@ -150,9 +173,10 @@ template <typename T>
 __device__ __forceinline__ void diag_sites(const T* __restrict__ mac, const DiagConsts& k, DiagRing<T>& ring, int b,
                                            int nblocks, double (&acc)[DIAG_NSUM], double& vmin, double& vmax) {
     const long long N = k.N, nxy = (long long)k.nx * k.ny;
-    const int gx = (k.nx + DIAG_TX - 1) / DIAG_TX, gy = (k.ny + DIAG_TY - 1) / DIAG_TY;
+    const int TX = 1 << k.ltx, TY = DIAG_NT >> k.ltx, EX = TX + 2, np = EX * (TY + 2);
+    const int gx = (k.nx + TX - 1) / TX, gy = (k.ny + TY - 1) / TY;
     const long long items = (long long)gx * gy * ((k.nz + k.chunk - 1) / k.chunk);
-    const int tid = threadIdx.x, tx = tid % DIAG_TX, ty = tid / DIAG_TX, p = (ty + 1) * DIAG_EX + tx + 1;
+    const int tid = threadIdx.x, tx = tid & (TX - 1), ty = tid >> k.ltx, p = (ty + 1) * EX + tx + 1;
     DiagAcc<T> a;
     a.v = a.dp = a.u[0] = a.u[1] = a.u[2] = a.ke = a.diss = a.in = a.out = 0.0;
     a.n = 0;
@@ -161,15 +185,15 @@ __device__ __forceinline__ void diag_sites(const T* __restrict__ mac, const Diag
     a.vmax = T(-INFINITY);
     for (long long it = b; it < items; it += nblocks) {
         const int bz = (int)(it / (gx * gy)), r = (int)(it - (long long)bz * gx * gy), by = r / gx, bx = r - by * gx;
-        const int x = bx * DIAG_TX + tx, y = by * DIAG_TY + ty;
+        const int x = bx * TX + tx, y = by * TY + ty;
         const int z0 = bz * k.chunk, z1 = min(z0 + k.chunk, k.nz);
         const bool act = x < k.nx && y < k.ny;
         const long long col = act ? x + (long long)k.nx * y : 0;
         long long off[2];  // this thread's ring positions tid, tid + DIAG_NT
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
-            const int q = tid + j * DIAG_NT, ey = q / DIAG_EX, ex = q - ey * DIAG_EX;
-            off[j] = (bx * DIAG_TX - 1 + ex + k.nx) % k.nx + (long long)k.nx * ((by * DIAG_TY - 1 + ey + k.ny) % k.ny);
+            const int q = tid + j * DIAG_NT, ey = q / EX, ex = q - ey * EX;
+            off[j] = (bx * TX - 1 + ex + k.nx) % k.nx + (long long)k.nx * ((by * TY - 1 + ey + k.ny) % k.ny);
         }
         T nu[2][3], nv = T(0), ndp = T(0);  // the plane in flight
         auto fetch = [&](int z) {
@@ -178,14 +202,14 @@ __device__ __forceinline__ void diag_sites(const T* __restrict__ mac, const Diag
             for (int j = 0; j < 2; ++j)
 #pragma unroll
                 for (int c = 0; c < 3; ++c)
-                    if (tid + j * DIAG_NT < DIAG_P) nu[j][c] = __ldg(pl + c * N + off[j]);
+                    if (tid + j * DIAG_NT < np) nu[j][c] = __ldg(pl + c * N + off[j]);
         };
         auto store = [&](int z) {
 #pragma unroll
             for (int j = 0; j < 2; ++j)
 #pragma unroll
                 for (int c = 0; c < 3; ++c)
-                    if (tid + j * DIAG_NT < DIAG_P) ring.u[z & 3][c][tid + j * DIAG_NT] = nu[j][c];
+                    if (tid + j * DIAG_NT < np) ring.u[z & 3][c][tid + j * DIAG_NT] = nu[j][c];
         };
         __syncthreads();  // the previous chunk's readers
         fetch(z0 - 1);
@@ -205,7 +229,7 @@ __device__ __forceinline__ void diag_sites(const T* __restrict__ mac, const Diag
                 nv = __ldg(mac + nxy * (z + 1) + col);
                 ndp = __ldg(mac + 4 * N + nxy * (z + 1) + col);
             }
-            if (act) diag_site(ring.u[(z - 1) & 3], ring.u[z & 3], ring.u[(z + 1) & 3], p, v, dp, k, z, a);
+            if (act) diag_site(ring.u[(z - 1) & 3], ring.u[z & 3], ring.u[(z + 1) & 3], p, EX, v, dp, k, z, a);
         }
         const double X = (double)x, Y = (double)y, WX = X * a.W, WY = Y * a.W;
         acc[8] += a.W;

@@ -13,6 +13,7 @@
 //    - kappag lap(phi) (chemical_potencial_cal, :998-1010; the 14-neighbour
 //    Laplacian of various_cal) and of |grad phi|^2.
 #include "dl_internal.cuh"
+#include "diag_site.cuh"
 
 #include <cufft.h>
 #include <math.h>
@@ -81,7 +82,7 @@ __global__ void __launch_bounds__(EN_THREADS) en_bin(const double* __restrict__ 
 
 // per-block partial sums of psi, mu and |grad phi|^2
 struct EnArgs {
-    int nx, ny, nz, chunk;
+    int nx, ny, nz, ltx, chunk;  // ltx, chunk: as in diag_site.cuh
     long long N;
     const void* mac;
     double phi_off, T, a, b, kappag, inv_lap, inv_grad;
@@ -96,23 +97,24 @@ struct EnArgs {
 // the 14 neighbours with products by c took 113), one reciprocal serves both
 // quotients, the stencil factors are applied to the sums. 128^3 FP32: 640 ->
 // 346 us, a third of it the logarithm.
-constexpr int EN_TX = 32, EN_TY = 8, EN_EX = EN_TX + 2, EN_P = EN_EX * (EN_TY + 2);
+static_assert(EN_THREADS == DIAG_NT, "the tiles of diag_site.cuh");
 template <typename T>
 __global__ void __launch_bounds__(EN_THREADS) en_free_energy(const EnArgs a) {
-    __shared__ double ring[4][EN_P];
+    __shared__ double ring[4][DIAG_P];
     const T* __restrict__ phi = (const T*)a.mac;
-    const int tid = threadIdx.x, tx = tid % EN_TX, ty = tid / EN_TX;
-    const int gx = (a.nx + EN_TX - 1) / EN_TX, gy = (a.ny + EN_TY - 1) / EN_TY, gz = (a.nz + a.chunk - 1) / a.chunk;
+    const int TX = 1 << a.ltx, TY = EN_THREADS >> a.ltx, EX = TX + 2, np = EX * (TY + 2);
+    const int tid = threadIdx.x, tx = tid & (TX - 1), ty = tid >> a.ltx;
+    const int gx = (a.nx + TX - 1) / TX, gy = (a.ny + TY - 1) / TY, gz = (a.nz + a.chunk - 1) / a.chunk;
     const long long nxy = (long long)a.nx * a.ny, items = (long long)gx * gy * gz;
-    const int k0 = (ty + 1) * EN_EX + tx + 1;
+    const int k0 = (ty + 1) * EX + tx + 1;
     double psi = 0.0, mu = 0.0, lap = 0.0, grad = 0.0;
     for (long long it = blockIdx.x; it < items; it += gridDim.x) {
         const int bz = (int)(it / (gx * gy)), r = (int)(it - (long long)bz * gx * gy), by = r / gx, bx = r - by * gx;
-        const int x0 = bx * EN_TX, y0 = by * EN_TY, z0 = bz * a.chunk, z1 = min(z0 + a.chunk, a.nz);
+        const int x0 = bx * TX, y0 = by * TY, z0 = bz * a.chunk, z1 = min(z0 + a.chunk, a.nz);
         long long off[2];
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
-            const int p = tid + j * EN_THREADS, ey = p / EN_EX, ex = p - ey * EN_EX;
+            const int p = tid + j * EN_THREADS, ey = p / EX, ex = p - ey * EX;
             const int x = (x0 - 1 + ex + a.nx) % a.nx, y = (y0 - 1 + ey + a.ny) % a.ny;
             off[j] = x + (long long)a.nx * y;
         }
@@ -120,7 +122,7 @@ __global__ void __launch_bounds__(EN_THREADS) en_free_energy(const EnArgs a) {
             const long long zo = nxy * (z < 0 ? z + a.nz : (z >= a.nz ? z - a.nz : z));
 #pragma unroll
             for (int j = 0; j < 2; ++j)
-                if (tid + j * EN_THREADS < EN_P) ring[z & 3][tid + j * EN_THREADS] = (double)__ldg(phi + zo + off[j]);
+                if (tid + j * EN_THREADS < np) ring[z & 3][tid + j * EN_THREADS] = (double)__ldg(phi + zo + off[j]);
         };
         const bool act = x0 + tx < a.nx && y0 + ty < a.ny;
         __syncthreads();  // the previous item's readers
@@ -138,12 +140,12 @@ __global__ void __launch_bounds__(EN_THREADS) en_free_energy(const EnArgs a) {
                 d[k] = vp - vm;
             };
             pair(0, c[1], c[-1]);
-            pair(1, c[EN_EX], c[-EN_EX]);
+            pair(1, c[EX], c[-EX]);
             pair(2, p[0], m[0]);
-            pair(3, p[EN_EX + 1], m[-EN_EX - 1]);   // c_7 = (+,+,+)
-            pair(4, p[EN_EX - 1], m[-EN_EX + 1]);   // c_8 = (-,+,+)
-            pair(5, p[-EN_EX + 1], m[EN_EX - 1]);   // c_9 = (+,-,+)
-            pair(6, m[EN_EX + 1], p[-EN_EX - 1]);   // c_10 = (+,+,-)
+            pair(3, p[EX + 1], m[-EX - 1]);   // c_7 = (+,+,+)
+            pair(4, p[EX - 1], m[-EX + 1]);   // c_8 = (-,+,+)
+            pair(5, p[-EX + 1], m[EX - 1]);   // c_9 = (+,-,+)
+            pair(6, m[EX + 1], p[-EX - 1]);   // c_10 = (+,+,-)
             const double v = c[0], ph = a.phi_off + v;
             lap += __fma_rn(-14.0, v, s);
             const double e = d[3] + d[4], f = d[5] + d[6], g = d[3] - d[4], h = d[5] - d[6];
@@ -247,17 +249,8 @@ int energy_diagnostics(dl_handle* h, dl_energy_diag* out, double* spectrum_host,
     a.inv_lap = 1.0 / (5.0 * h->P.ds * h->P.ds);
     a.inv_grad = 1.0 / (10.0 * h->P.ds);
     a.part = h->en_buf + h->en_bytes / sizeof(double) - 3 * EN_BLOCKS;
-    // planes per item: the even split of nz with the least rounds x (planes + the two ring planes' loads)
-    const long long tiles = (long long)((h->nx + EN_TX - 1) / EN_TX) * ((h->ny + EN_TY - 1) / EN_TY);
-    double cost = 1e300;
-    for (int m = 1; m <= h->nz; ++m) {
-        const int c = (h->nz + m - 1) / m;
-        const double t = (double)((tiles * ((h->nz + c - 1) / c) + EN_BLOCKS - 1) / EN_BLOCKS) * (c + 0.7);
-        if (t < cost) {
-            cost = t;
-            a.chunk = c;
-        }
-    }
+    a.ltx = diag_tile(a.nx, a.ny);
+    a.chunk = diag_chunk(diag_tiles(a.nx, a.ny, a.ltx), a.nz, EN_BLOCKS, 0.7);
     if (fast) DL_LAUNCH(h, false, (en_free_energy<float><<<EN_BLOCKS, EN_THREADS, 0, h->stream>>>(a)));
     else DL_LAUNCH(h, false, (en_free_energy<double><<<EN_BLOCKS, EN_THREADS, 0, h->stream>>>(a)));
     DL_CUDA(h, cudaGetLastError());

@@ -139,7 +139,7 @@ static int reduce_any(dl_handle* h, const T* d_mac, double phi_off, double p_off
     RedArgs a;
     memset(&a, 0, sizeof(a));
     diag_consts(h, phi_off, p_off, a.k);
-    a.k.chunk = diag_chunk(h->nx, h->ny, h->nz, RED_BLOCKS);
+    diag_march(a.k, RED_BLOCKS);
     a.part = h->d_diag;
     DL_LAUNCH(h, false, reduce_partials<T><<<RED_BLOCKS, RED_THREADS, 0, h->stream>>>(d_mac, a));
     DL_LAUNCH(h, false, reduce_final<<<NPART, 32, 0, h->stream>>>(h->d_diag, RED_BLOCKS, h->d_diag + RED_BLOCKS * NPART));

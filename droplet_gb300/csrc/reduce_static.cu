@@ -219,7 +219,7 @@ static int reduce_static_any(dl_handle* h, const T* d_mac, double phi_off, doubl
     RsArgs a;
     memset(&a, 0, sizeof(a));
     diag_consts(h, phi_off, p_off, a.k);
-    a.k.chunk = diag_chunk(h->nx, h->ny, h->nz, nblocks);
+    diag_march(a.k, nblocks);
     // the arrival counter starts at zero whatever an earlier launch left
     DL_CUDA(h, cudaMemsetAsync(scratch + (size_t)RS_MAX_BLOCKS * RS_NPART + RS_NPART, 0, sizeof(unsigned long long),
                                h->stream));

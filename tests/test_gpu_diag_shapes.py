@@ -18,7 +18,7 @@ from oracle import np_energy
 
 pytestmark = pytest.mark.gpu
 
-SHAPES = [(3, 3, 3), (5, 9, 40), (33, 7, 21), (32, 8, 64), (40, 17, 130), (7, 100, 3), (129, 3, 5), (65, 33, 37),
+SHAPES = [(3, 3, 3), (5, 9, 40), (48, 10, 19), (33, 7, 21), (32, 8, 64), (40, 17, 130), (7, 100, 3), (129, 3, 5), (65, 33, 37),
           (330, 250, 5)]
 
 
