@@ -113,6 +113,12 @@ DL_HD double div_by(double x, const DivBy& d) {
     return div_markstein(x, d.y, d.zh);
 }
 
+// x / 3: DIV_SHORT with 1/3 and the rest of it, 1/3 - RN(1/3) = 2^-54 / 3
+DL_HD double div3(double x) {
+    if (!div_numerator_ok(x)) return div_general(x, 3.0);
+    return div_short(x, 1.0 / 3.0, 0x1.5555555555555p-56);
+}
+
 // the way for divisor y (host)
 inline DivBy make_div_by(double y) {
     DivBy d = {y, 0.0, 0.0, DIV_GENERAL};

@@ -852,12 +852,6 @@ __global__ void __launch_bounds__(POPS_NT) pops_to_host(const FastArgs a, double
     pops_run_out(ga + s0 * Q, buf, n);
 }
 
-// x / 3 as the IEEE division rounds it, in two FP64 instructions (DIV_SHORT of div_by.cuh)
-__device__ __forceinline__ double third(double x) {
-    if (!div_numerator_ok(x)) return div_general(x, 3.0);
-    return __fma_rn(x, 1.0 / 3.0, __dmul_rn(x, 0x1.5555555555555p-56));
-}
-
 // full f, g (direction fastest, doubles) -> moments and stored populations; the
 // FP64 pipe is the bound (15 divisions and 45 products by c before)
 template <typename ST, bool RES>
@@ -880,7 +874,7 @@ __global__ void __launch_bounds__(POPS_NT) pops_from_host(const FastArgs a, cons
     for (int i = 0; i < Q; ++i) {
         const double fv = fb[threadIdx.x * Q + i], gv = gb[threadIdx.x * Q + i];
         ph += fv;
-        pp += third(gv);
+        pp += div3(gv);
         if (cx(i)) m1 = cx(i) > 0 ? m1 + gv : m1 - gv;
         if (cy(i)) m2 = cy(i) > 0 ? m2 + gv : m2 - gv;
         if (cz(i)) m3 = cz(i) > 0 ? m3 + gv : m3 - gv;

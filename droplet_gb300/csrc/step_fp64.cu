@@ -61,15 +61,6 @@ struct Fp64Args {
     long long step;
 };
 
-// 1/3 and the rest of it: 3 is DIV_SHORT
-constexpr double THIRD_HI = 1.0 / 3.0;
-constexpr double THIRD_LO = 0x1.5555555555555p-56;  // 1/3 - THIRD_HI = 2^-54 / 3
-
-__device__ __forceinline__ double div3(double x) {
-    if (!div_numerator_ok(x)) return div_general(x, 3.0);
-    return div_fma(x, THIRD_HI, x * THIRD_LO);
-}
-
 // classification by the bits: a comparison would take the FP64 pipe
 __device__ __forceinline__ bool finite_bits(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
 __device__ __forceinline__ bool nan_bits(double v) {
