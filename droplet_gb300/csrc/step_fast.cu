@@ -721,11 +721,12 @@ __global__ void __launch_bounds__(PROJ_NT, 4) sp_project_fast(const FastArgs a) 
 }
 
 // the projection of the fused step as a launch of its own, over chunks of
-// BAND_CHUNK planes whatever the step's lz: the same sums in the same order as
-// a step whose blocks march BAND_CHUNK planes, so that the two-phase results do
-// not depend on how the step is cut: FP16 storage turns any change of rounding in
-// the force into one FP16 quantum here and there, which spreads, and FP32
-// checkpoints after a few steps are otherwise 1e-9 apart.
+// BAND_CHUNK planes where lz is chosen automatically and is another number: the
+// same sums in the same order as a step whose blocks march BAND_CHUNK planes, so
+// that the two-phase results do not depend on how the step is cut: FP16 storage
+// turns any change of rounding in the force into one FP16 quantum here and there,
+// which spreads, and FP32 checkpoints after a few steps are otherwise 1e-9 apart.
+// An explicit lz keeps the sums in the step, grouped by its own marches.
 constexpr int BAND_CHUNK = 32;
 __global__ void __launch_bounds__(NT) project_chunks(const FastArgs a) {
     __shared__ __align__(16) float scr[PT_SCRATCH];
